@@ -54,14 +54,14 @@ class BlockLU:
         for b, M in enumerate(blocks):
             self.block(b).copy_(torch.as_tensor(np.asarray(M, dtype=np.float64)))
 
-    panel = 0  # panel width of the factorisation (0: size-based default)
+    panel = 0  # panel width of the factorisation (0: chosen by size; blocks up to 256: the tensor-core kernel)
 
     def tune_panel(self, reps: int = 3) -> int:
-        """Time the panel widths 8/16/32 on the current blocks and keep the
-        fastest (restores the blocks afterwards)."""
+        """Time the default (0) and the panel widths 8/16/32 on the current
+        blocks and keep the fastest (restores the blocks afterwards)."""
         saved = self.A.clone()
         best, best_t = 0, float("inf")
-        for p in (8, 16, 32):
+        for p in (0, 8, 16, 32):
             from ._lib import F3DError
             try:
                 self.A.copy_(saved)
