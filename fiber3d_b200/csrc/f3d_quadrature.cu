@@ -6,7 +6,7 @@
 // body/body.py:104-107).
 //
 // The reference loops over triangles in Python (about 5 ms each).  Here the
-// whole computation is eight kernels on one stream:
+// whole computation is nine kernels on one stream:
 //   1. quad_prep: per triangle, sorted vertices, unit normal and midpoint;
 //      its three edges go into a device hash table (key = i * n + j).
 //   2. quad_edges: per triangle edge, the partner triangle from the table and
@@ -15,16 +15,17 @@
 //      selected exactly among the float-rounded squared distances held in
 //      shared memory, ties resolved on the double distances, then index.
 //      The nodes go in tiles of 24576, the best 80 carried from tile to tile.
-//   4. quad_triangle: per triangle, the projection onto the triangle's plane
+//   4. quad_geometry: per triangle, the projection onto the triangle's plane
 //      (:162-236), the exact integrals of r^7 (:262-309) and of the degree-7
 //      monomials (:473-622, here by Gauss-Legendre on Green's-theorem line
-//      integrals) and the 116 x 116 saddle-point solve (:334-336),
-//      Gauss-Jordan elimination with partial pivoting held in registers
-//      (16 x 16 threads, an 8 x 8 tile each), the right-hand side carried
-//      along as column 116; then the area-element distortion (:431-447).
+//      integrals) and the area-element distortion (:431-447); quad_triangle:
+//      the 116 x 116 saddle-point solve (:334-336), LU with partial pivoting in
+//      shared memory, 16 columns at a time, the trailing update on the FP64
+//      tensor cores, the right-hand side carried along.
 //   5. quad_count / quad_scan / quad_fill / quad_sum: the per-node sum of the
 //      triangle weights in triangle order (:460-468), deterministic.
 #include <algorithm>
+#include <climits>
 
 #include "f3d_common.cuh"
 
@@ -63,7 +64,8 @@ struct QuadWs {
   long long *hkey;  // hash keys (-1 empty)
   int32_t *hid;     // 2 per key: stacked edge ids (-1 empty)
   int32_t *nni;     // ntri x 80
-  double *wt;       // ntri x 80
+  double *wt;       // ntri x 80: the area-element factors, then the triangles' weights
+  double *rec;      // kTriRec per triangle of a chunk
   int32_t *count;   // n + 1 (exclusive offsets after the scan)
   int32_t *cursor;  // n
   int32_t *entry;   // ntri x 80
@@ -385,338 +387,454 @@ __device__ __forceinline__ double rbf_right_triangle(double a, double b) {
 
 __device__ __forceinline__ double sgn(double x) { return x > 0.0 ? 1.0 : (x < 0.0 ? -1.0 : 0.0); }
 
-constexpr int kTriThreads = 256;
+// The projection and the right-hand side of each triangle t of [t_lo, t_hi):
+// the projected centres (80 x 2) and the integrals (116) to its record, the
+// area-element factors to its 80 entries of w.wt.  Mostly serial chains of
+// divisions, square roots and asinh over at most 116 threads, so it is a
+// kernel of its own with many CTAs per SM (0.43 ms at 24500 triangles); inside
+// the elimination kernel the chains ran with nothing beside them.
+constexpr int kGeoThreads = 128;
+constexpr int kTriRec = 2 * kQuadNbr + kQuadDim;
 
-struct TriShared {
-  double c[kQuadNbr][2];         // projected, shifted centres
-  double pm[kQuadNbr][kQuadPoly];  // monomials of the centres
-  double rhs[kQuadDim];
-  double dist[kQuadNbr];
-  double l[128];
-  double u[128];
-  double ys[128];
-  double x[kQuadDim];
-  double piv[kQuadDim];
-  double recip[kQuadDim];
-  int order[kQuadDim];
-  int where[128];
+struct GeoShared {
+  double c[kQuadNbr][2];  // projected, shifted centres
+  double l[kQuadNbr], ys[kQuadNbr];
   double xp[3], rot[9], shift[2], v[3][2], height;
-  int prow;
 };
 
-// The pivot row's entries in register columns KB..7 go to S.u (u_j = 0 for
-// j <= k in column block KB).
-template <int KB>
-__device__ __forceinline__ void stage_row(const double (&row)[8], TriShared &S, int tx, int k) {
-  const int j = tx + 16 * KB;
-  S.u[j] = j > k ? row[KB] : 0.0;
-#pragma unroll
-  for (int b = KB + 1; b < 8; ++b) S.u[tx + 16 * b] = row[b];
-}
-
-// Pivot of column k (register column C of the threads with tx == k % 16,
-// one half-warp): the largest |a_ik| over the rows not yet pivoted (`used`:
-// bit a for row ty + 16 a), the first in the current row order on ties
-// (LAPACK's choice); its lane stores the pivot and its reciprocal, lane 0
-// exchanges the rows.
-template <int C>
-__device__ __forceinline__ void pivot_column(const double (&M)[8][8], TriShared &S, unsigned used, int k, int ty,
-                                             int tx, int *err) {
-  const unsigned half = (tx & 1) ? 0xffff0000u : 0x0000ffffu;
-  double best = -1.0, mine = 0.0;
-  int ia = -1;
-#pragma unroll
-  for (int a = 0; a < 8; ++a) {
-    const int i = ty + 16 * a;
-    if (i < kQuadDim && !((used >> a) & 1u)) {
-      const double av = fabs(M[a][C]);
-      if (av > best || (av == best && S.where[i] < S.where[ty + 16 * ia])) best = av, ia = a, mine = M[a][C];
-    }
-  }
-  int bpos = ia >= 0 ? S.where[ty + 16 * ia] : 0x7fffffff;
-  const int my_pos = bpos;
-  const double my_recip = 1.0 / mine;  // formed while the reduction runs
-#pragma unroll
-  for (int o = 8; o > 0; o >>= 1) {
-    const double ob = __shfl_xor_sync(half, best, o, 16);
-    const int op = __shfl_xor_sync(half, bpos, o, 16);
-    if (ob > best || (ob == best && op < bpos)) best = ob, bpos = op;
-  }
-  if (my_pos == bpos && bpos != 0x7fffffff) {
-    S.piv[k] = mine;
-    S.recip[k] = my_recip;
-  }
-  __syncwarp(half);
-  if (ty == 0) {
-    if (!(best > 0.0)) {
-      record_error(err, F3D_ERR_SINGULAR);
-      bpos = k;
-      S.piv[k] = 1.0;
-      S.recip[k] = 1.0;
-    }
-    const int rk = S.order[k], rp = S.order[bpos];
-    S.order[k] = rp, S.order[bpos] = rk;
-    S.where[rp] = k, S.where[rk] = bpos;
-    S.prow = rp;
-  }
-}
-
-// Gauss-Jordan steps k = 16 KB .. 16 KB + ncol - 1 (the pivot of step k
-// already chosen): every row but the pivot row loses l_i = a_ik / a_pk times
-// the pivot row, so that after the last step row order[k] holds u_kk in
-// column k and y_k in column 116, and x_k = y_k / u_kk (no back
-// substitution).  Columns up to k are left as they are.  The pivot column is
-// register column KB of the threads with tx == k % 16: a static index, so it
-// never leaves registers; column blocks before KB are skipped.  After its own
-// update, the half-warp that owns column k + 1 chooses that column's pivot
-// while the other warps finish theirs.
-template <int KB>
-__device__ __forceinline__ void gj_columns(double (&M)[8][8], TriShared &S, unsigned &used, int ncol, int ty, int tx,
-                                           int *err) {
-  for (int kk = 0; kk < ncol; ++kk) {
-    const int k = 16 * KB + kk;
-    const int prow = S.prow;
-    if (ty == (prow & 15)) used |= 1u << (prow >> 4);
-    if (tx == kk) {
-      const double r = S.recip[k];
-#pragma unroll
-      for (int a = 0; a < 8; ++a) {
-        const int i = ty + 16 * a;
-        S.l[i] = (i < kQuadDim && i != prow) ? M[a][KB] * r : 0.0;
-      }
-    }
-    if (ty == (prow & 15)) {
-      switch (prow >> 4) {
-        case 0: stage_row<KB>(M[0], S, tx, k); break;
-        case 1: stage_row<KB>(M[1], S, tx, k); break;
-        case 2: stage_row<KB>(M[2], S, tx, k); break;
-        case 3: stage_row<KB>(M[3], S, tx, k); break;
-        case 4: stage_row<KB>(M[4], S, tx, k); break;
-        case 5: stage_row<KB>(M[5], S, tx, k); break;
-        case 6: stage_row<KB>(M[6], S, tx, k); break;
-        default: stage_row<KB>(M[7], S, tx, k); break;
-      }
-    }
-    __syncthreads();
-    double ur[8 - KB];
-#pragma unroll
-    for (int b = KB; b < 8; ++b) ur[b - KB] = S.u[tx + 16 * b];
-#pragma unroll
-    for (int a = 0; a < 8; ++a) {
-      const double lr = -S.l[ty + 16 * a];
-#pragma unroll
-      for (int b = KB; b < 8; ++b) M[a][b] = fma(lr, ur[b - KB], M[a][b]);
-    }
-    if (k + 1 < kQuadDim) {
-      if (kk + 1 < 16) {
-        if (tx == kk + 1) pivot_column<KB>(M, S, used, k + 1, ty, tx, err);
-      } else if constexpr (KB < 7) {
-        if (tx == 0) pivot_column<KB + 1>(M, S, used, k + 1, ty, tx, err);
-      }
-    }
-    __syncthreads();
-  }
-}
-
-__global__ void __launch_bounds__(kTriThreads, 1) quad_triangle_kernel(const double *__restrict__ X,
-                                                                       const double *__restrict__ grad, int ntri,
-                                                                       QuadWs w, int *err) {
-  __shared__ TriShared S;
+__global__ void __launch_bounds__(kGeoThreads) quad_geometry_kernel(const double *__restrict__ X,
+                                                                    const double *__restrict__ grad, int t_lo,
+                                                                    QuadWs w) {
+  __shared__ GeoShared S;
   const int tid = threadIdx.x;
-  const int ty = tid & 15, tx = tid >> 4;  // rows ty + 16a, columns tx + 16b
-  for (int t = blockIdx.x; t < ntri; t += gridDim.x) {
-    const int *tv = w.tri + 3 * t;
-    const double *nrm = w.tnorm + 3 * t;
-    const int32_t *nb = w.nni + static_cast<int64_t>(t) * kQuadNbr;
-    if (tid == 0) {
-      // projection point (:162-201)
-      double A[3], B[3], C[3], AB[3], BC[3], CA[3];
-      for (int c = 0; c < 3; ++c) {
-        A[c] = X[3 * tv[0] + c], B[c] = X[3 * tv[1] + c], C[c] = X[3 * tv[2] + c];
-        AB[c] = __dsub_rn(B[c], A[c]), BC[c] = __dsub_rn(C[c], B[c]), CA[c] = __dsub_rn(A[c], C[c]);
-      }
-      const double *nAB = w.enorm + 9 * t, *nCA = nAB + 3, *nBC = nAB + 6;
-      double nOAB[3], nOBC[3], nOCA[3], vOA[3];
-      cross_rn(nAB, AB, nOAB);
-      cross_rn(nBC, BC, nOBC);
-      cross_rn(nCA, CA, nOCA);
-      cross_rn(nOAB, nOCA, vOA);
-      const double tA = __ddiv_rn(dot3_rn(nOBC, AB), dot3_rn(nOBC, vOA));
-      for (int c = 0; c < 3; ++c) S.xp[c] = __dadd_rn(A[c], __dmul_rn(tA, vOA[c]));
-      // rotation taking the normal to +z (:210-220)
-      const double rxy = __dsqrt_rn(__dadd_rn(__dmul_rn(nrm[0], nrm[0]), __dmul_rn(nrm[1], nrm[1])));
-      if (rxy < kDblEps) {
-        for (int i = 0; i < 9; ++i) S.rot[i] = (i % 4 == 0) ? 1.0 : 0.0;
-      } else {
-        const double nn = __dsqrt_rn(dot3_rn(nrm, nrm));
-        const double r1[9] = {__ddiv_rn(nrm[2], nn), 0.0, -__ddiv_rn(rxy, nn), 0.0, 1.0, 0.0,
-                              __ddiv_rn(rxy, nn), 0.0, __ddiv_rn(nrm[2], nn)};
-        const double r2[9] = {__ddiv_rn(nrm[0], rxy), __ddiv_rn(nrm[1], rxy), 0.0, -__ddiv_rn(nrm[1], rxy),
-                              __ddiv_rn(nrm[0], rxy), 0.0, 0.0, 0.0, 1.0};
-        for (int i = 0; i < 3; ++i)
-          for (int j = 0; j < 3; ++j)
-            S.rot[3 * i + j] = __dadd_rn(__dadd_rn(__dmul_rn(r1[3 * i], r2[j]), __dmul_rn(r1[3 * i + 1], r2[3 + j])),
-                                         __dmul_rn(r1[3 * i + 2], r2[6 + j]));
-      }
-      double d[3];
-      for (int c = 0; c < 3; ++c) d[c] = __dsub_rn(w.mid[3 * t + c], S.xp[c]);
-      S.shift[0] = dot3_rn(S.rot, d);
-      S.shift[1] = dot3_rn(S.rot + 3, d);
-      const double *V[3] = {A, B, C};
-      for (int r = 0; r < 3; ++r) {
-        for (int c = 0; c < 3; ++c) d[c] = __dsub_rn(V[r][c], S.xp[c]);
-        S.v[r][0] = __dsub_rn(dot3_rn(S.rot, d), S.shift[0]);
-        S.v[r][1] = __dsub_rn(dot3_rn(S.rot + 3, d), S.shift[1]);
-      }
+  const int t = t_lo + static_cast<int>(blockIdx.x);
+  double *rec = w.rec + static_cast<int64_t>(blockIdx.x) * kTriRec;
+  const int *tv = w.tri + 3 * t;
+  const double *nrm = w.tnorm + 3 * t;
+  const int32_t *nb = w.nni + static_cast<int64_t>(t) * kQuadNbr;
+  if (tid == 0) {
+    // projection point (:162-201)
+    double A[3], B[3], C[3], AB[3], BC[3], CA[3];
+    for (int c = 0; c < 3; ++c) {
+      A[c] = X[3 * tv[0] + c], B[c] = X[3 * tv[1] + c], C[c] = X[3 * tv[2] + c];
+      AB[c] = __dsub_rn(B[c], A[c]), BC[c] = __dsub_rn(C[c], B[c]), CA[c] = __dsub_rn(A[c], C[c]);
     }
-    __syncthreads();
-    if (tid < kQuadNbr) {
-      // project neighbour tid into the plane (:225-236)
-      const int j = nb[tid];
-      double Q[3], d[3], p[3];
-      for (int c = 0; c < 3; ++c) Q[c] = X[3 * j + c];
-      const double A0 = X[3 * tv[0]], A1 = X[3 * tv[0] + 1], A2 = X[3 * tv[0] + 2];
-      const double num = __dadd_rn(__dadd_rn(__dmul_rn(nrm[0], __dsub_rn(A0, Q[0])), __dmul_rn(nrm[1], __dsub_rn(A1, Q[1]))),
-                                   __dmul_rn(nrm[2], __dsub_rn(A2, Q[2])));
-      for (int c = 0; c < 3; ++c) d[c] = __dsub_rn(Q[c], S.xp[c]);
-      const double mult = __ddiv_rn(num, dot3_rn(nrm, d));
-      for (int c = 0; c < 3; ++c) p[c] = __dsub_rn(__dadd_rn(Q[c], __dmul_rn(mult, d[c])), S.xp[c]);
-      const double u0 = dot3_rn(S.rot, p), u1 = dot3_rn(S.rot + 3, p), u2 = dot3_rn(S.rot + 6, p);
-      if (tid == 0) S.height = u2;
-      const double cx = __dsub_rn(u0, S.shift[0]), cy = __dsub_rn(u1, S.shift[1]);
-      S.c[tid][0] = cx, S.c[tid][1] = cy;
-      // monomials by the reference's recursion (:324-329)
-      double *pm = S.pm[tid];
-      pm[0] = 1.0;
-      for (int dg = 1; dg <= kQuadOrder; ++dg)
-        for (int k = 0; k <= dg; ++k)
-          pm[dg * (dg + 1) / 2 + k] = (k >= (dg + 1) / 2) ? __dmul_rn(cy, pm[(dg - 1) * dg / 2 + k - 1])
-                                                          : __dmul_rn(cx, pm[(dg - 1) * dg / 2 + k]);
-      // area-element distortion (:431-442)
-      const double *g = grad + 3 * j;
-      const double gn = __dsqrt_rn(dot3_rn(g, g));
-      const double nv = __dsqrt_rn(dot3_rn(d, d));
-      double vh[3], ns[3];
-      for (int c = 0; c < 3; ++c) vh[c] = __ddiv_rn(d[c], nv), ns[c] = __ddiv_rn(g[c], gn);
-      const double pn = __dsqrt_rn(dot3_rn(nrm, nrm));
-      double pu[3];
-      for (int c = 0; c < 3; ++c) pu[c] = __ddiv_rn(nrm[c], pn);
-      S.ys[tid] = __ddiv_rn(dot3_rn(pu, vh), dot3_rn(ns, vh));  // ratio of the normal projections
-      S.l[tid] = nv;
+    const double *nAB = w.enorm + 9 * t, *nCA = nAB + 3, *nBC = nAB + 6;
+    double nOAB[3], nOBC[3], nOCA[3], vOA[3];
+    cross_rn(nAB, AB, nOAB);
+    cross_rn(nBC, BC, nOBC);
+    cross_rn(nCA, CA, nOCA);
+    cross_rn(nOAB, nOCA, vOA);
+    const double tA = __ddiv_rn(dot3_rn(nOBC, AB), dot3_rn(nOBC, vOA));
+    for (int c = 0; c < 3; ++c) S.xp[c] = __dadd_rn(A[c], __dmul_rn(tA, vOA[c]));
+    // rotation taking the normal to +z (:210-220)
+    const double rxy = __dsqrt_rn(__dadd_rn(__dmul_rn(nrm[0], nrm[0]), __dmul_rn(nrm[1], nrm[1])));
+    if (rxy < kDblEps) {
+      for (int i = 0; i < 9; ++i) S.rot[i] = (i % 4 == 0) ? 1.0 : 0.0;
+    } else {
+      const double nn = __dsqrt_rn(dot3_rn(nrm, nrm));
+      const double r1[9] = {__ddiv_rn(nrm[2], nn), 0.0, -__ddiv_rn(rxy, nn), 0.0, 1.0, 0.0,
+                            __ddiv_rn(rxy, nn), 0.0, __ddiv_rn(nrm[2], nn)};
+      const double r2[9] = {__ddiv_rn(nrm[0], rxy), __ddiv_rn(nrm[1], rxy), 0.0, -__ddiv_rn(nrm[1], rxy),
+                            __ddiv_rn(nrm[0], rxy), 0.0, 0.0, 0.0, 1.0};
+      for (int i = 0; i < 3; ++i)
+        for (int j = 0; j < 3; ++j)
+          S.rot[3 * i + j] = __dadd_rn(__dadd_rn(__dmul_rn(r1[3 * i], r2[j]), __dmul_rn(r1[3 * i + 1], r2[3 + j])),
+                                       __dmul_rn(r1[3 * i + 2], r2[6 + j]));
     }
-    __syncthreads();
-    if (tid < kQuadNbr) {
-      const double cx = __dadd_rn(S.c[tid][0], S.shift[0]), cy = __dadd_rn(S.c[tid][1], S.shift[1]);
-      const double R = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(cx, cx), __dmul_rn(cy, cy)), __dmul_rn(S.height, S.height)));
-      const double rr = __ddiv_rn(S.l[tid], R);
-      S.dist[tid] = fabs(__dmul_rn(S.ys[tid], __dmul_rn(rr, rr)));
-      // exact integral of r^7 centred at this node over the triangle (:262-309)
-      const double c0 = S.c[tid][0], c1 = S.c[tid][1];
-      const double(*V)[2] = S.v;
-      const double sabc = sgn(__dadd_rn(__dmul_rn(__dsub_rn(V[0][1], V[1][1]), __dsub_rn(V[2][0], V[0][0])),
-                                        __dmul_rn(__dsub_rn(V[1][0], V[0][0]), __dsub_rn(V[2][1], V[0][1]))));
-      double irbf = 0.0;
-      for (int s = 0; s < 3; ++s) {
-        const double *p1 = V[s], *p2 = V[(s + 1) % 3];
-        const double ex = __dsub_rn(p2[0], p1[0]), ey = __dsub_rn(p2[1], p1[1]);
-        const double m = __ddiv_rn(__dadd_rn(__dmul_rn(__dsub_rn(c0, p1[0]), ex), __dmul_rn(__dsub_rn(c1, p1[1]), ey)),
-                                   __dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey)));
-        const double fx = __dadd_rn(__dmul_rn(m, ex), p1[0]), fy = __dadd_rn(__dmul_rn(m, ey), p1[1]);
-        const double sg1 = sabc * sgn(__dadd_rn(__dmul_rn(__dsub_rn(c1, p1[1]), __dsub_rn(fx, c0)),
-                                                __dmul_rn(__dsub_rn(p1[0], c0), __dsub_rn(fy, c1))));
-        const double sg2 = sabc * sgn(__dadd_rn(__dmul_rn(__dsub_rn(c1, fy), __dsub_rn(p2[0], c0)),
-                                                __dmul_rn(__dsub_rn(fx, c0), __dsub_rn(p2[1], c1))));
-        const double ax = __dsub_rn(c0, fx), ay = __dsub_rn(c1, fy);
-        const double alpha = __dsqrt_rn(__dadd_rn(__dmul_rn(ax, ax), __dmul_rn(ay, ay)));
-        const double b1x = __dsub_rn(fx, p1[0]), b1y = __dsub_rn(fy, p1[1]);
-        const double b2x = __dsub_rn(fx, p2[0]), b2y = __dsub_rn(fy, p2[1]);
-        const double beta1 = __dsqrt_rn(__dadd_rn(__dmul_rn(b1x, b1x), __dmul_rn(b1y, b1y)));
-        const double beta2 = __dsqrt_rn(__dadd_rn(__dmul_rn(b2x, b2x), __dmul_rn(b2y, b2y)));
-        const double tiny = kEpsMult * kDblEps;
-        if (alpha > tiny && beta1 > tiny) irbf += sg1 * rbf_right_triangle(alpha, beta1);
-        if (alpha > tiny && beta2 > tiny) irbf += sg2 * rbf_right_triangle(alpha, beta2);
-      }
-      S.rhs[tid] = irbf;
-    } else if (tid < kQuadDim) {
-      // polynomial moment m = tid - 80 of the triangle (Green's theorem,
-      // Gauss-Legendre along each side)
-      const int m = tid - kQuadNbr;
-      int dg = 0;
-      while ((dg + 1) * (dg + 2) / 2 <= m) ++dg;
-      const int k = m - dg * (dg + 1) / 2, a = dg - k;
-      const double(*V)[2] = S.v;
-      const double sabc = sgn(__dadd_rn(__dmul_rn(__dsub_rn(V[0][1], V[1][1]), __dsub_rn(V[2][0], V[0][0])),
-                                        __dmul_rn(__dsub_rn(V[1][0], V[0][0]), __dsub_rn(V[2][1], V[0][1]))));
-      double acc = 0.0;
-      for (int s = 0; s < 3; ++s) {
-        const double *p1 = V[s], *p2 = V[(s + 1) % 3];
-        const double ex = p2[0] - p1[0], ey = p2[1] - p1[1];
-        double line = 0.0;
-        for (int q = 0; q < 6; ++q) {
-          const double tq = 0.5 * (kGlX[q] + 1.0);
-          const double xq = p1[0] + tq * ex, yq = p1[1] + tq * ey;
-          double v = 0.5 * kGlW[q];
-          for (int e = 0; e <= a; ++e) v *= xq;
-          for (int e = 0; e < k; ++e) v *= yq;
-          line += v;
-        }
-        acc += ey * line / (a + 1);
-      }
-      S.rhs[tid] = sabc * acc;
+    double d[3];
+    for (int c = 0; c < 3; ++c) d[c] = __dsub_rn(w.mid[3 * t + c], S.xp[c]);
+    S.shift[0] = dot3_rn(S.rot, d);
+    S.shift[1] = dot3_rn(S.rot + 3, d);
+    const double *V[3] = {A, B, C};
+    for (int r = 0; r < 3; ++r) {
+      for (int c = 0; c < 3; ++c) d[c] = __dsub_rn(V[r][c], S.xp[c]);
+      S.v[r][0] = __dsub_rn(dot3_rn(S.rot, d), S.shift[0]);
+      S.v[r][1] = __dsub_rn(dot3_rn(S.rot + 3, d), S.shift[1]);
     }
+  }
+  __syncthreads();
+  if (tid < kQuadNbr) {
+    // project neighbour tid into the plane (:225-236)
+    const int j = nb[tid];
+    double Q[3], d[3], p[3];
+    for (int c = 0; c < 3; ++c) Q[c] = X[3 * j + c];
+    const double A0 = X[3 * tv[0]], A1 = X[3 * tv[0] + 1], A2 = X[3 * tv[0] + 2];
+    const double num = __dadd_rn(__dadd_rn(__dmul_rn(nrm[0], __dsub_rn(A0, Q[0])), __dmul_rn(nrm[1], __dsub_rn(A1, Q[1]))),
+                                 __dmul_rn(nrm[2], __dsub_rn(A2, Q[2])));
+    for (int c = 0; c < 3; ++c) d[c] = __dsub_rn(Q[c], S.xp[c]);
+    const double mult = __ddiv_rn(num, dot3_rn(nrm, d));
+    for (int c = 0; c < 3; ++c) p[c] = __dsub_rn(__dadd_rn(Q[c], __dmul_rn(mult, d[c])), S.xp[c]);
+    const double u0 = dot3_rn(S.rot, p), u1 = dot3_rn(S.rot + 3, p), u2 = dot3_rn(S.rot + 6, p);
+    if (tid == 0) S.height = u2;
+    const double cx = __dsub_rn(u0, S.shift[0]), cy = __dsub_rn(u1, S.shift[1]);
+    S.c[tid][0] = cx, S.c[tid][1] = cy;
+    rec[2 * tid] = cx, rec[2 * tid + 1] = cy;
+    // area-element distortion (:431-442)
+    const double *g = grad + 3 * j;
+    const double gn = __dsqrt_rn(dot3_rn(g, g));
+    const double nv = __dsqrt_rn(dot3_rn(d, d));
+    double vh[3], ns[3];
+    for (int c = 0; c < 3; ++c) vh[c] = __ddiv_rn(d[c], nv), ns[c] = __ddiv_rn(g[c], gn);
+    const double pn = __dsqrt_rn(dot3_rn(nrm, nrm));
+    double pu[3];
+    for (int c = 0; c < 3; ++c) pu[c] = __ddiv_rn(nrm[c], pn);
+    S.ys[tid] = __ddiv_rn(dot3_rn(pu, vh), dot3_rn(ns, vh));  // ratio of the normal projections
+    S.l[tid] = nv;
+  }
+  __syncthreads();
+  if (tid < kQuadNbr) {
+    const double cx = __dadd_rn(S.c[tid][0], S.shift[0]), cy = __dadd_rn(S.c[tid][1], S.shift[1]);
+    const double R = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(cx, cx), __dmul_rn(cy, cy)), __dmul_rn(S.height, S.height)));
+    const double rr = __ddiv_rn(S.l[tid], R);
+    w.wt[static_cast<int64_t>(t) * kQuadNbr + tid] = fabs(__dmul_rn(S.ys[tid], __dmul_rn(rr, rr)));
+    // exact integral of r^7 centred at this node over the triangle (:262-309)
+    const double c0 = S.c[tid][0], c1 = S.c[tid][1];
+    const double(*V)[2] = S.v;
+    const double sabc = sgn(__dadd_rn(__dmul_rn(__dsub_rn(V[0][1], V[1][1]), __dsub_rn(V[2][0], V[0][0])),
+                                      __dmul_rn(__dsub_rn(V[1][0], V[0][0]), __dsub_rn(V[2][1], V[0][1]))));
+    double irbf = 0.0;
+    for (int s = 0; s < 3; ++s) {
+      const double *p1 = V[s], *p2 = V[(s + 1) % 3];
+      const double ex = __dsub_rn(p2[0], p1[0]), ey = __dsub_rn(p2[1], p1[1]);
+      const double m = __ddiv_rn(__dadd_rn(__dmul_rn(__dsub_rn(c0, p1[0]), ex), __dmul_rn(__dsub_rn(c1, p1[1]), ey)),
+                                 __dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey)));
+      const double fx = __dadd_rn(__dmul_rn(m, ex), p1[0]), fy = __dadd_rn(__dmul_rn(m, ey), p1[1]);
+      const double sg1 = sabc * sgn(__dadd_rn(__dmul_rn(__dsub_rn(c1, p1[1]), __dsub_rn(fx, c0)),
+                                              __dmul_rn(__dsub_rn(p1[0], c0), __dsub_rn(fy, c1))));
+      const double sg2 = sabc * sgn(__dadd_rn(__dmul_rn(__dsub_rn(c1, fy), __dsub_rn(p2[0], c0)),
+                                              __dmul_rn(__dsub_rn(fx, c0), __dsub_rn(p2[1], c1))));
+      const double ax = __dsub_rn(c0, fx), ay = __dsub_rn(c1, fy);
+      const double alpha = __dsqrt_rn(__dadd_rn(__dmul_rn(ax, ax), __dmul_rn(ay, ay)));
+      const double b1x = __dsub_rn(fx, p1[0]), b1y = __dsub_rn(fy, p1[1]);
+      const double b2x = __dsub_rn(fx, p2[0]), b2y = __dsub_rn(fy, p2[1]);
+      const double beta1 = __dsqrt_rn(__dadd_rn(__dmul_rn(b1x, b1x), __dmul_rn(b1y, b1y)));
+      const double beta2 = __dsqrt_rn(__dadd_rn(__dmul_rn(b2x, b2x), __dmul_rn(b2y, b2y)));
+      const double tiny = kEpsMult * kDblEps;
+      if (alpha > tiny && beta1 > tiny) irbf += sg1 * rbf_right_triangle(alpha, beta1);
+      if (alpha > tiny && beta2 > tiny) irbf += sg2 * rbf_right_triangle(alpha, beta2);
+    }
+    rec[2 * kQuadNbr + tid] = irbf;
+  } else if (tid < kQuadDim) {
+    // polynomial moment m = tid - 80 of the triangle (Green's theorem,
+    // Gauss-Legendre along each side)
+    const int m = tid - kQuadNbr;
+    int dg = 0;
+    while ((dg + 1) * (dg + 2) / 2 <= m) ++dg;
+    const int k = m - dg * (dg + 1) / 2, a = dg - k;
+    const double(*V)[2] = S.v;
+    const double sabc = sgn(__dadd_rn(__dmul_rn(__dsub_rn(V[0][1], V[1][1]), __dsub_rn(V[2][0], V[0][0])),
+                                      __dmul_rn(__dsub_rn(V[1][0], V[0][0]), __dsub_rn(V[2][1], V[0][1]))));
+    double acc = 0.0;
+    for (int s = 0; s < 3; ++s) {
+      const double *p1 = V[s], *p2 = V[(s + 1) % 3];
+      const double ex = p2[0] - p1[0], ey = p2[1] - p1[1];
+      double line = 0.0;
+      for (int q = 0; q < 6; ++q) {
+        const double tq = 0.5 * (kGlX[q] + 1.0);
+        const double xq = p1[0] + tq * ex, yq = p1[1] + tq * ey;
+        double v = 0.5 * kGlW[q];
+        for (int e = 0; e <= a; ++e) v *= xq;
+        for (int e = 0; e < k; ++e) v *= yq;
+        line += v;
+      }
+      acc += ey * line / (a + 1);
+    }
+    rec[2 * kQuadNbr + tid] = sabc * acc;
+  }
+}
+
+// The 116 x 116 saddle-point system of each triangle: LU with partial pivoting
+// (LAPACK's choice of pivots), the right-hand side carried along as column
+// 116, and back substitution.
+//
+// The chain of 116 pivots bounds it (the 0.5 Mflop of a triangle are 8000
+// tensor-core cycles), so two triangles share an SM: a CTA is 256 threads, at
+// most 128 registers and the matrix in 110 KB of shared memory, with
+// everything else in the 5.5 KB that two such CTAs leave.  That is why
+//  * panels are 16 columns whose rows (one per thread) go through the 16
+//    pivots in registers, with one barrier per pivot;
+//  * U12 and L21 stay where they are in the matrix, and the trailing update
+//    (16 x 16 outputs per warp at a time, on the FP64 tensor cores) reads its
+//    operands there;
+//  * rows are never exchanged: `phys` maps positions to rows, a pivot is the
+//    first position of largest magnitude, and the trailing rows are gathered
+//    by position.
+// Row stride 118 doubles: a thread's 16-byte reads of its own row are free of
+// bank conflicts, the tensor-core fragments' two-way at worst.
+// The panels' transformations are not applied as explicit products (blocked
+// Gauss-Jordan, which needs no back substitution): these systems have
+// condition numbers near 1e17, and on a 200-node sphere of radius 0.5 that
+// moved the weights by 7e-8.
+// 24500 triangles: 7.7 ms, against 27.9 ms for unblocked Gauss-Jordan with the
+// matrix in the registers of one CTA per SM, two barriers per pivot.
+constexpr int kTriThreads = 256;
+constexpr int kTriWarps = kTriThreads / 32;
+constexpr int kTriS = kQuadDim + 2;  // row stride: 116 columns, the right-hand side, one of padding
+constexpr int kTriPW = 4;            // warps with panel rows
+constexpr size_t kTriSmem = static_cast<size_t>(kQuadDim) * kTriS * sizeof(double);
+
+struct TriShared {
+  __align__(16) double cand[2][kTriPW][16];  // each warp's best row, by step parity
+  __align__(16) double l11[16][16];          // column-major unit lower triangle of the panel
+  double rcp[2][kTriPW];                     // the reciprocal of its candidate
+  double c[kQuadNbr][2];                     // projected centres; then the unknowns
+  unsigned hi[2][kTriPW], lo[2][kTriPW];     // the candidate's key
+  int pos[2][kTriPW];
+  int phys[kQuadDim];                        // row at each position
+};
+
+// sqrt(x^7) = x^3 sqrt(x) (x >= 0; NaN below): the cube as a two-term sum, so
+// that the result has the square root's rounding and its own.
+__device__ __forceinline__ double sqrt_pow7(double x) {
+  const double t = x * x, te = fma(x, x, -t);
+  const double c = t * x, ce = fma(te, x, fma(t, x, -c));
+  const double s = sqrt(x), p = c * s;
+  return p + fma(ce, s, fma(c, s, -p));
+}
+
+// Pivot k = c0 + jj of the panel (jj static) on the rows in v.
+template <int jj>
+__device__ __forceinline__ void tri_pivot(double (&v)[16], TriShared &S, int k, bool &done, int &pos, int lane,
+                                          int warp, int *err) {
+  constexpr int par = jj & 1;
+  // this row's candidacy: 0 none, 1 a NaN, else the bits of |a| plus 2
+  const double mag = fabs(v[jj]);
+  const unsigned long long key =
+      done ? 0ull : (mag != mag ? 1ull : static_cast<unsigned long long>(__double_as_longlong(mag)) + 2ull);
+  const double rcp = 1.0 / v[jj];  // beside the search
+  const unsigned hi = static_cast<unsigned>(key >> 32), lo = static_cast<unsigned>(key);
+  const unsigned hmax = __reduce_max_sync(0xffffffffu, hi);
+  bool best = hi == hmax;
+  if (__popc(__ballot_sync(0xffffffffu, best)) > 1) {
+    const unsigned lmax = __reduce_max_sync(0xffffffffu, best ? lo : 0u);
+    best = best && lo == lmax;
+    const int pmin = __reduce_min_sync(0xffffffffu, best ? pos : INT_MAX);
+    best = best && pos == pmin;
+  }
+  if (best) {  // one lane (a warp with no candidate left posts key 0, which never wins)
+    S.hi[par][warp] = hi;
+    S.lo[par][warp] = lo;
+    S.pos[par][warp] = pos;
+    S.rcp[par][warp] = rcp;
+#pragma unroll
+    for (int j = jj & ~1; j < 16; j += 2)
+      *reinterpret_cast<double2 *>(&S.cand[par][warp][j]) = make_double2(v[j], v[j + 1]);
+  }
+  asm volatile("bar.sync 1, %0;" ::"n"(32 * kTriPW) : "memory");
+  // the best warp: lane w looks at warp w's post
+  const unsigned wh = S.hi[par][lane & (kTriPW - 1)];
+  const unsigned whmax = __reduce_max_sync(0xffffffffu, wh);
+  unsigned ties = __ballot_sync(0xffffffffu, wh == whmax) & ((1u << kTriPW) - 1u);
+  int bw = __ffs(ties) - 1;
+  while (ties &= ties - 1u) {  // equal leading words: the rest of the key, then the position
+    const int w = __ffs(ties) - 1;
+    const unsigned lw = S.lo[par][w], lb = S.lo[par][bw];
+    if (lw > lb || (lw == lb && S.pos[par][w] < S.pos[par][bw])) bw = w;
+  }
+  const int pp = S.pos[par][bw];
+  const double *prow = S.cand[par][bw];
+  const double d = prow[jj], rd = S.rcp[par][bw];
+  if (pos == pp) {  // the pivot row
+    pos = k;
+    done = true;
+    if (!(fabs(d) > 0.0)) {  // zero or not a number: an error; go on as if the pivot were 1
+      record_error(err, F3D_ERR_SINGULAR);
+      v[jj] = 1.0;
+    }
+  } else if (pos == k) {
+    pos = pp;
+  }
+  if (!done) {
+    const double l0 = v[jj] * rd;  // v / d with one residual correction (Markstein)
+    const double l = fma(fma(-l0, d, v[jj]), rd, l0);
+    v[jj] = l;
+#pragma unroll
+    for (int j = jj + 1; j < 16; ++j) v[j] = fma(-l, prow[j], v[j]);
+  }
+}
+
+template <int jj>
+__device__ __forceinline__ void tri_panel(double (&v)[16], TriShared &S, int c0, int nb, bool &done, int &pos,
+                                          int lane, int warp, int *err) {
+  if constexpr (jj < 16) {
+    if (jj >= nb) return;
+    tri_pivot<jj>(v, S, c0 + jj, done, pos, lane, warp, err);
+    tri_panel<jj + 1>(v, S, c0, nb, done, pos, lane, warp, err);
+  }
+}
+
+__global__ void __launch_bounds__(kTriThreads, 2) quad_triangle_kernel(int t_lo, int count, QuadWs w, int *err) {
+  extern __shared__ __align__(16) double tri_smem[];
+  __shared__ TriShared S;
+  double *X = tri_smem;  // [116][kTriS]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int it = blockIdx.x; it < count; it += gridDim.x) {
+    const double *rec = w.rec + static_cast<int64_t>(it) * kTriRec;
+    for (int i = tid; i < 2 * kQuadNbr; i += kTriThreads) (&S.c[0][0])[i] = rec[i];
     if (tid < kQuadDim) {
-      S.order[tid] = tid;
+      *reinterpret_cast<double2 *>(X + tid * kTriS + kQuadRhsCol) = make_double2(rec[2 * kQuadNbr + tid], 0.0);
+      S.phys[tid] = tid;
     }
-    if (tid < 128) S.where[tid] = tid;
+    __syncthreads();
+    // [Phi P; P^T 0]
+    if (tid < kQuadNbr) {  // monomials by the reference's recursion (:324-329)
+      const double cx = S.c[tid][0], cy = S.c[tid][1];
+      double below[kQuadOrder + 1], row[kQuadOrder + 1];
+      row[0] = 1.0;
+#pragma unroll
+      for (int dg = 0; dg <= kQuadOrder; ++dg) {
+        if (dg > 0) {
+#pragma unroll
+          for (int k = 0; k <= dg; ++k)
+            row[k] = (k >= (dg + 1) / 2) ? __dmul_rn(cy, below[k - 1]) : __dmul_rn(cx, below[k]);
+        }
+#pragma unroll
+        for (int k = 0; k <= dg; ++k) {
+          const int m = kQuadNbr + dg * (dg + 1) / 2 + k;
+          X[tid * kTriS + m] = row[k];
+          X[m * kTriS + tid] = row[k];
+          below[k] = row[k];
+        }
+      }
+    } else {
+      for (int e = tid - kQuadNbr; e < kQuadPoly * kQuadPoly; e += kTriThreads - kQuadNbr)
+        X[(kQuadNbr + e / kQuadPoly) * kTriS + kQuadNbr + e % kQuadPoly] = 0.0;
+    }
+    for (int e = tid; e < kQuadNbr * kQuadNbr; e += kTriThreads) {
+      const int i = e / kQuadNbr, j = e % kQuadNbr;
+      const double xi = S.c[i][0], yi = S.c[i][1], xj = S.c[j][0], yj = S.c[j][1];
+      const double di = __dadd_rn(__dmul_rn(xi, xi), __dmul_rn(yi, yi));
+      const double dj = __dadd_rn(__dmul_rn(xj, xj), __dmul_rn(yj, yj));
+      const double ip = __dadd_rn(__dmul_rn(xi, xj), __dmul_rn(yi, yj));
+      X[i * kTriS + j] = sqrt_pow7(__dsub_rn(__dadd_rn(dj, di), __dmul_rn(2.0, ip)));
+    }
     __syncthreads();
 
-    // augmented matrix [Phi P rhs; P^T 0 rhs] in registers, padded to 128 x 128
-    double M[8][8];
+    for (int c0 = 0; c0 < kQuadDim; c0 += 16) {
+      const int nb = min(16, kQuadDim - c0), m = kQuadDim - c0;
+      if (warp < kTriPW) {
+        const bool live = tid < m;
+        bool done = !live;
+        int pos = live ? c0 + tid : INT_MAX;
+        const int row = live ? S.phys[pos] : 0;
+        double v[16];
+        double *x = X + row * kTriS + c0;
 #pragma unroll
-    for (int a = 0; a < 8; ++a) {
-      const int i = ty + 16 * a;
-#pragma unroll
-      for (int b = 0; b < 8; ++b) {
-        const int j = tx + 16 * b;
-        double v = 0.0;
-        if (j == kQuadRhsCol) {
-          v = i < kQuadDim ? S.rhs[i] : 0.0;
-        } else if (i < kQuadNbr && j < kQuadNbr) {
-          const double xi = S.c[i][0], yi = S.c[i][1], xj = S.c[j][0], yj = S.c[j][1];
-          const double di = __dadd_rn(__dmul_rn(xi, xi), __dmul_rn(yi, yi));
-          const double dj = __dadd_rn(__dmul_rn(xj, xj), __dmul_rn(yj, yj));
-          const double ip = __dadd_rn(__dmul_rn(xi, xj), __dmul_rn(yi, yj));
-          const double r2 = __dsub_rn(__dadd_rn(dj, di), __dmul_rn(2.0, ip));
-          v = sqrt(pow(r2, 7.0));
-        } else if (i < kQuadNbr && j < kQuadDim) {
-          v = S.pm[i][j - kQuadNbr];
-        } else if (i < kQuadDim && j < kQuadNbr) {
-          v = S.pm[j][i - kQuadNbr];
+        for (int j = 0; j < 16; j += 2) {
+          double2 a = make_double2(0.0, 0.0);
+          if (j < nb) a = *reinterpret_cast<const double2 *>(x + j);
+          v[j] = a.x;
+          v[j + 1] = a.y;
         }
-        M[a][b] = v;
+        tri_panel<0>(v, S, c0, nb, done, pos, lane, warp, err);
+        if (live) {
+#pragma unroll
+          for (int j = 0; j < 16; j += 2)
+            if (j < nb) *reinterpret_cast<double2 *>(x + j) = make_double2(v[j], v[j + 1]);
+          S.phys[pos] = row;
+          if (pos < c0 + nb) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) S.l11[j][pos - c0] = v[j];
+          }
+        }
+      }
+      __syncthreads();
+      // U12 = L11^-1 A12, a column per thread (the right-hand side the last)
+      const int cs = c0 + nb;
+      if (tid <= kQuadRhsCol - cs) {
+        double u[16];
+        double *xc = X + cs + tid;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) u[i] = i < nb ? xc[S.phys[min(c0 + i, kQuadDim - 1)] * kTriS] : 0.0;
+#pragma unroll
+        for (int i = 0; i < 15; ++i) {
+          if (i >= nb) break;
+#pragma unroll
+          for (int r = i + 1; r < 16; ++r)
+            if (r < nb) u[r] = fma(-S.l11[i][r], u[i], u[r]);
+        }
+#pragma unroll
+        for (int i = 1; i < 16; ++i)
+          if (i < nb) xc[S.phys[min(c0 + i, kQuadDim - 1)] * kTriS] = u[i];
+      }
+      __syncthreads();
+      // A22 -= L21 U12 (panels before the last have 16 columns)
+      const int g = lane >> 2, t = lane & 3;
+      const int m2 = kQuadDim - cs, rts = (m2 + 15) / 16, cts = (m2 + 1 + 15) / 16;
+      for (int it2 = warp; m2 > 0 && it2 < rts * cts; it2 += kTriWarps) {
+        const int rt = it2 % rts, c = cs + 16 * (it2 / rts);
+        const int p0 = 16 * rt + g, p1 = p0 + 8;
+        double *x0 = X + S.phys[cs + min(p0, m2 - 1)] * kTriS, *x1 = X + S.phys[cs + min(p1, m2 - 1)] * kTriS;
+        double af[8], bf[2][4];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) af[q] = -((q & 1) ? x1 : x0)[c0 + t + 4 * (q >> 1)];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const double *u = X + S.phys[c0 + t + 4 * j] * kTriS;
+#pragma unroll
+          for (int ni = 0; ni < 2; ++ni) bf[ni][j] = u[min(c + 8 * ni + g, kQuadRhsCol)];
+        }
+#pragma unroll
+        for (int ni = 0; ni < 2; ++ni) {
+          const int cc = c + 8 * ni + 2 * t;  // this lane's two columns (the second may be the padding)
+          const bool cv = cc <= kQuadRhsCol;
+          double2 o0 = make_double2(0.0, 0.0), o1 = o0;
+          if (cv) {
+            o0 = *reinterpret_cast<const double2 *>(x0 + cc);
+            o1 = *reinterpret_cast<const double2 *>(x1 + cc);
+          }
+          double dd[4] = {o0.x, o0.y, o1.x, o1.y};
+          mma_f64_16816(dd, af, bf[ni]);
+          if (cv) {
+            if (p0 < m2) *reinterpret_cast<double2 *>(x0 + cc) = make_double2(dd[0], dd[1]);
+            if (p1 < m2) *reinterpret_cast<double2 *>(x1 + cc) = make_double2(dd[2], dd[3]);
+          }
+        }
+      }
+      __syncthreads();
+    }
+    // back substitution by blocks of 16: the warp that holds the block's
+    // positions solves its triangle, then every earlier position takes the
+    // block's unknowns out (x stays in S.c)
+    if (warp < kTriPW) {
+      double *xs = &S.c[0][0];
+      const int k = tid;
+      const double *u = X + S.phys[min(k, kQuadDim - 1)] * kTriS;
+      double y = k < kQuadDim ? u[kQuadRhsCol] : 0.0;
+      const double d = k < kQuadDim ? u[k] : 1.0, rd = 1.0 / d;
+      for (int c0 = (kQuadDim - 1) / 16 * 16; c0 >= 0; c0 -= 16) {
+        const int nb = min(16, kQuadDim - c0);
+        if (warp == c0 / 32) {
+          for (int j = nb - 1; j >= 0; --j) {
+            const double q = y * rd;  // y / d with one residual correction (Markstein)
+            const double x = __shfl_sync(0xffffffffu, fma(fma(-q, d, y), rd, q), (c0 + j) & 31);
+            if (k == c0 + j) {
+              xs[k] = x;
+            } else if (k >= c0 && k < c0 + j) {
+              y = fma(-u[c0 + j], x, y);
+            }
+          }
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * kTriPW) : "memory");
+        if (k < c0) {
+          double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+          for (int j = 0; j < 16; j += 2) {
+            if (j < nb) {
+              const double2 a = *reinterpret_cast<const double2 *>(u + c0 + j);
+              s0 = fma(a.x, xs[c0 + j], s0);
+              s1 = fma(a.y, xs[c0 + j + 1], s1);
+            }
+          }
+          y -= s0 + s1;
+        }
+      }
+      if (tid < kQuadNbr) {
+        double *o = w.wt + static_cast<int64_t>(t_lo + it) * kQuadNbr + tid;
+        *o = __dmul_rn(xs[tid], *o);
       }
     }
-
-    // Gauss-Jordan elimination with partial pivoting (rows stay in place;
-    // order/where hold the row exchanges), the right-hand side carried along
-    unsigned used = 0;
-    if (tx == 0) pivot_column<0>(M, S, used, 0, ty, tx, err);
-    __syncthreads();
-    gj_columns<0>(M, S, used, 16, ty, tx, err);
-    gj_columns<1>(M, S, used, 16, ty, tx, err);
-    gj_columns<2>(M, S, used, 16, ty, tx, err);
-    gj_columns<3>(M, S, used, 16, ty, tx, err);
-    gj_columns<4>(M, S, used, 16, ty, tx, err);
-    gj_columns<5>(M, S, used, 16, ty, tx, err);
-    gj_columns<6>(M, S, used, 16, ty, tx, err);
-    gj_columns<7>(M, S, used, kQuadDim - 112, ty, tx, err);
-    if (tx == (kQuadRhsCol & 15)) {
-#pragma unroll
-      for (int a = 0; a < 8; ++a) S.ys[ty + 16 * a] = M[a][kQuadRhsCol >> 4];
-    }
-    __syncthreads();
-    if (tid < kQuadNbr) S.x[tid] = S.ys[S.order[tid]] / S.piv[tid];
-    if (tid < kQuadNbr) w.wt[static_cast<int64_t>(t) * kQuadNbr + tid] = __dmul_rn(S.x[tid], S.dist[tid]);
     __syncthreads();
   }
 }
@@ -810,6 +928,9 @@ __global__ void __launch_bounds__(32 * kSumWarps) quad_sum_kernel(int n, QuadWs 
   if (lane == 0) weights[i] = s;
 }
 
+// The systems go through in chunks, so that their records stay within 72 MB.
+constexpr int64_t kTriChunk = 32768;
+
 static int hash_bits(int64_t ntri) {
   int b = 6;
   while ((1ll << b) < 4 * ntri) ++b;
@@ -834,6 +955,7 @@ static size_t quad_layout(int64_t n, int64_t ntri, QuadWs *w, char *base) {
   q.hid = reinterpret_cast<int32_t *>(take(sizeof(int32_t) * 2 * H));
   q.nni = reinterpret_cast<int32_t *>(take(sizeof(int32_t) * kQuadNbr * ntri));
   q.wt = reinterpret_cast<double *>(take(sizeof(double) * kQuadNbr * ntri));
+  q.rec = reinterpret_cast<double *>(take(sizeof(double) * kTriRec * std::min(ntri, kTriChunk)));
   q.count = reinterpret_cast<int32_t *>(take(sizeof(int32_t) * (n + 1)));
   q.cursor = reinterpret_cast<int32_t *>(take(sizeof(int32_t) * n));
   q.entry = reinterpret_cast<int32_t *>(take(sizeof(int32_t) * kQuadNbr * ntri));
@@ -901,8 +1023,19 @@ int f3d_surface_quadrature(const double *nodes, int64_t n, const int32_t *triang
   const int64_t knn_grid = std::min<int64_t>((ntri + 1) / 2, static_cast<int64_t>(per_sm) * f3d::sm_count());
   f3d::quad_knn_kernel<<<static_cast<unsigned>(knn_grid), f3d::kKnnThreads, knn_smem, st>>>(nodes, nn, w.mid, nt,
                                                                                             tile, w.nni, err);
-  const int64_t tri_grid = std::min<int64_t>(ntri, f3d::sm_count());
-  f3d::quad_triangle_kernel<<<static_cast<unsigned>(tri_grid), f3d::kTriThreads, 0, st>>>(nodes, gradient, nt, w, err);
+  static bool tri_attr[64] = {false};
+  if (!tri_attr[dev]) {
+    if (cudaFuncSetAttribute(f3d::quad_triangle_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(f3d::kTriSmem)) != cudaSuccess)
+      return F3D_ERR_CUDA;
+    tri_attr[dev] = true;
+  }
+  for (int64_t lo = 0; lo < ntri; lo += f3d::kTriChunk) {
+    const int count = static_cast<int>(std::min(ntri - lo, f3d::kTriChunk));
+    f3d::quad_geometry_kernel<<<count, f3d::kGeoThreads, 0, st>>>(nodes, gradient, static_cast<int>(lo), w);
+    const int grid = std::min(count, 2 * f3d::sm_count());
+    f3d::quad_triangle_kernel<<<grid, f3d::kTriThreads, f3d::kTriSmem, st>>>(static_cast<int>(lo), count, w, err);
+  }
   const int64_t m = f3d::kQuadNbr * ntri;
   f3d::quad_count_kernel<<<static_cast<unsigned>((m + 255) / 256), 256, 0, st>>>(m, w);
   f3d::quad_scan_kernel<<<1, 1024, 0, st>>>(nn, w);
