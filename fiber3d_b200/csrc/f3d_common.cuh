@@ -106,6 +106,18 @@ __device__ __forceinline__ void mma_f64_16816(double (&d)[4], const double (&a)[
         "d"(b[1]), "d"(b[2]), "d"(b[3]));
 }
 
+// 1/x for the pivot: the hardware approximation (rcp.approx.ftz.f64, about
+// 2^-22 relative error) refined by one third-order Newton step
+// y1 = y0 (1 + e + e^2), e = 1 - x y0, whose error is O(e^3): within an ulp
+// or so of the correctly rounded quotient, in 4 dependent operations.
+// Pivots below the normal range are reported as zero pivots by the caller.
+__device__ __forceinline__ double reciprocal(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+
 __device__ __forceinline__ void record_error(int *err, int code) {
   if (err) atomicCAS(err, 0, code);
 }

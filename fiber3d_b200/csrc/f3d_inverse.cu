@@ -45,18 +45,6 @@ struct InvShape {
   static constexpr int kThreads = kColTiles * kRowTiles;
 };
 
-// 1/x for the pivot: the hardware approximation (rcp.approx.ftz.f64, about
-// 2^-22 relative error) refined by one third-order Newton step
-// y1 = y0 (1 + e + e^2), e = 1 - x y0, whose error is O(e^3): within an ulp
-// or so of the correctly rounded quotient, in 4 dependent operations.
-// Pivots below the normal range are reported as zero pivots by the caller.
-__device__ __forceinline__ double reciprocal(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x, y, 1.0);
-  return fma(y, fma(e, e, e), y);
-}
-
 // Step k = kb + M of the Gauss-Jordan sweep on the register tiles.
 // Column k is published to shared memory and zeroed in the tiles; the pivot
 // row is read back with its column-k entry taken as 1, so that one update

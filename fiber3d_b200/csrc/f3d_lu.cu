@@ -249,10 +249,10 @@ __global__ void __launch_bounds__(kLuThreads) batched_lu_factor_kernel(const LuA
 // SM, whose pivot chains overlap.  (128 threads with two rows each: 1.95 ms
 // on the blocks below; every thread scanning the warps' keys and forming the
 // pivot's reciprocal after the barrier: 1.54 ms.)  Measured on 2000 blocks of
-// 64-256 rows (7.2 Gflop): 1.40 ms, against 5.95 ms for the kernel below
+// 64-256 rows (7.2 Gflop): 1.37 ms, against 5.95 ms for the kernel below
 // with its default panel of 32, 2.38 ms with 16 and 3.19 ms with 8; on 2000
-// blocks of 128 rows 0.68 ms against 1.54 ms (16).  One block of 256 rows
-// alone takes 0.31 ms, 0.99 ms before.
+// blocks of 128 rows 0.67 ms against 1.54 ms (16).  One block of 256 rows
+// alone takes 0.30 ms, 0.99 ms before.
 constexpr int kLtThreads = 256;
 constexpr int kLtWarps = kLtThreads / 32;
 constexpr int kLtNB = 16;
@@ -321,10 +321,10 @@ __device__ __forceinline__ void lt_factor_one(double *__restrict__ A, int n, int
         const double mag = fabs(v[jj]);
         const unsigned long long key =
             done ? 0ull : (mag != mag ? 1ull : static_cast<unsigned long long>(__double_as_longlong(mag)) + 2ull);
-        // the candidate's reciprocal, beside the search: l = v / d is formed
-        // from it with one residual correction (Markstein); pivots near the
-        // ends of the range divide instead
-        const double rcp = 1.0 / v[jj];
+        // the candidate's reciprocal, beside the search (no branch whatever the
+        // row holds): l = v / d is formed from it with one residual correction
+        // (Markstein); pivots near the ends of the range divide instead
+        const double rcp = reciprocal(v[jj]);
         const unsigned hi = static_cast<unsigned>(key >> 32), lo = static_cast<unsigned>(key);
         const unsigned hmax = __reduce_max_sync(0xffffffffu, hi);
         bool best = hi == hmax;

@@ -559,14 +559,17 @@ __global__ void __launch_bounds__(kGeoThreads) quad_geometry_kernel(const double
 //    operands there;
 //  * rows are never exchanged: `phys` maps positions to rows, a pivot is the
 //    first position of largest magnitude, and the trailing rows are gathered
-//    by position.
+//    by position;
+//  * half of the warps work on a panel; the others meanwhile apply the panel
+//    before to the columns after it (all first apply it to this panel's).
 // Row stride 118 doubles: a thread's 16-byte reads of its own row are free of
 // bank conflicts, the tensor-core fragments' two-way at worst.
 // The panels' transformations are not applied as explicit products (blocked
 // Gauss-Jordan, which needs no back substitution): these systems have
 // condition numbers near 1e17, and on a 200-node sphere of radius 0.5 that
 // moved the weights by 7e-8.
-// 24500 triangles: 7.7 ms, against 27.9 ms for unblocked Gauss-Jordan with the
+// 24500 triangles: 7.2 ms (7.7 without the look-ahead and with quotients on
+// the chain of back substitution), against 27.9 ms for unblocked Gauss-Jordan with the
 // matrix in the registers of one CTA per SM, two barriers per pivot.
 constexpr int kTriThreads = 256;
 constexpr int kTriWarps = kTriThreads / 32;
@@ -579,9 +582,11 @@ struct TriShared {
   __align__(16) double l11[16][16];          // column-major unit lower triangle of the panel
   double rcp[2][kTriPW];                     // the reciprocal of its candidate
   double c[kQuadNbr][2];                     // projected centres; then the unknowns
-  unsigned hi[2][kTriPW], lo[2][kTriPW];     // the candidate's key
+  __align__(16) unsigned hi[2][kTriPW];      // the candidate's key
+  unsigned lo[2][kTriPW];
   int pos[2][kTriPW];
-  int phys[kQuadDim];                        // row at each position
+  int phys[2][kQuadDim];                     // row at each position still to be reduced, by panel parity
+  int fin[kQuadDim];                         // row of each pivot
 };
 
 // sqrt(x^7) = x^3 sqrt(x) (x >= 0; NaN below): the cube as a two-term sum, so
@@ -622,15 +627,17 @@ __device__ __forceinline__ void tri_pivot(double (&v)[16], TriShared &S, int k, 
       *reinterpret_cast<double2 *>(&S.cand[par][warp][j]) = make_double2(v[j], v[j + 1]);
   }
   asm volatile("bar.sync 1, %0;" ::"n"(32 * kTriPW) : "memory");
-  // the best warp: lane w looks at warp w's post
-  const unsigned wh = S.hi[par][lane & (kTriPW - 1)];
-  const unsigned whmax = __reduce_max_sync(0xffffffffu, wh);
-  unsigned ties = __ballot_sync(0xffffffffu, wh == whmax) & ((1u << kTriPW) - 1u);
-  int bw = __ffs(ties) - 1;
-  while (ties &= ties - 1u) {  // equal leading words: the rest of the key, then the position
-    const int w = __ffs(ties) - 1;
-    const unsigned lw = S.lo[par][w], lb = S.lo[par][bw];
-    if (lw > lb || (lw == lb && S.pos[par][w] < S.pos[par][bw])) bw = w;
+  // the best warp
+  const uint4 h = *reinterpret_cast<const uint4 *>(S.hi[par]);
+  const unsigned top = max(max(h.x, h.y), max(h.z, h.w));
+  int bw = h.x == top ? 0 : (h.y == top ? 1 : (h.z == top ? 2 : 3));
+  if ((h.x == top) + (h.y == top) + (h.z == top) + (h.w == top) > 1) {
+    // equal leading words: the rest of the key, then the position
+    for (int w = bw + 1; w < kTriPW; ++w) {
+      if (S.hi[par][w] != top) continue;
+      const unsigned lw = S.lo[par][w], lb = S.lo[par][bw];
+      if (lw > lb || (lw == lb && S.pos[par][w] < S.pos[par][bw])) bw = w;
+    }
   }
   const int pp = S.pos[par][bw];
   const double *prow = S.cand[par][bw];
@@ -646,8 +653,7 @@ __device__ __forceinline__ void tri_pivot(double (&v)[16], TriShared &S, int k, 
     pos = pp;
   }
   if (!done) {
-    const double l0 = v[jj] * rd;  // v / d with one residual correction (Markstein)
-    const double l = fma(fma(-l0, d, v[jj]), rd, l0);
+    const double l = v[jj] * rd;
     v[jj] = l;
 #pragma unroll
     for (int j = jj + 1; j < 16; ++j) v[j] = fma(-l, prow[j], v[j]);
@@ -674,7 +680,7 @@ __global__ void __launch_bounds__(kTriThreads, 2) quad_triangle_kernel(int t_lo,
     for (int i = tid; i < 2 * kQuadNbr; i += kTriThreads) (&S.c[0][0])[i] = rec[i];
     if (tid < kQuadDim) {
       *reinterpret_cast<double2 *>(X + tid * kTriS + kQuadRhsCol) = make_double2(rec[2 * kQuadNbr + tid], 0.0);
-      S.phys[tid] = tid;
+      S.phys[0][tid] = tid;
     }
     __syncthreads();
     // [Phi P; P^T 0]
@@ -711,13 +717,52 @@ __global__ void __launch_bounds__(kTriThreads, 2) quad_triangle_kernel(int t_lo,
     }
     __syncthreads();
 
-    for (int c0 = 0; c0 < kQuadDim; c0 += 16) {
+    // The update by panel c0 of the columns [c, ce), c a multiple of 16 past
+    // cs: items of 16 x 16 outputs to warps w0, w0 + 1, ...
+    auto update = [&](int c0, const int *phys, int c_lo, int ce, int w0) {
+      const int g = lane >> 2, t = lane & 3;
+      const int cs = c0 + 16, m2 = kQuadDim - cs, rts = (m2 + 15) / 16, cts = (ce - c_lo + 15) / 16;
+      for (int it2 = warp - w0; it2 < rts * cts; it2 += kTriWarps - w0) {
+        const int rt = it2 % rts, c = c_lo + 16 * (it2 / rts);
+        const int p0 = 16 * rt + g, p1 = p0 + 8;
+        double *x0 = X + phys[cs + min(p0, m2 - 1)] * kTriS, *x1 = X + phys[cs + min(p1, m2 - 1)] * kTriS;
+        double af[8], bf[2][4];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) af[q] = -((q & 1) ? x1 : x0)[c0 + t + 4 * (q >> 1)];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const double *u = X + S.fin[c0 + t + 4 * j] * kTriS;
+#pragma unroll
+          for (int ni = 0; ni < 2; ++ni) bf[ni][j] = u[min(c + 8 * ni + g, kQuadRhsCol)];
+        }
+#pragma unroll
+        for (int ni = 0; ni < 2; ++ni) {
+          const int cc = c + 8 * ni + 2 * t;  // this lane's two columns (the second may be the padding)
+          const bool cv = cc < ce;
+          double2 o0 = make_double2(0.0, 0.0), o1 = o0;
+          if (cv) {
+            o0 = *reinterpret_cast<const double2 *>(x0 + cc);
+            o1 = *reinterpret_cast<const double2 *>(x1 + cc);
+          }
+          double dd[4] = {o0.x, o0.y, o1.x, o1.y};
+          mma_f64_16816(dd, af, bf[ni]);
+          if (cv) {
+            if (p0 < m2) *reinterpret_cast<double2 *>(x0 + cc) = make_double2(dd[0], dd[1]);
+            if (p1 < m2) *reinterpret_cast<double2 *>(x1 + cc) = make_double2(dd[2], dd[3]);
+          }
+        }
+      }
+    };
+    for (int c0 = 0, par = 0; c0 < kQuadDim; c0 += 16, par ^= 1) {
       const int nb = min(16, kQuadDim - c0), m = kQuadDim - c0;
+      // warps 0-3: the panel, from the row order of parity par to the other;
+      // warps 4-7 meanwhile: the previous panel's update of the columns after
+      // this one
       if (warp < kTriPW) {
         const bool live = tid < m;
         bool done = !live;
         int pos = live ? c0 + tid : INT_MAX;
-        const int row = live ? S.phys[pos] : 0;
+        const int row = live ? S.phys[par][pos] : 0;
         double v[16];
         double *x = X + row * kTriS + c0;
 #pragma unroll
@@ -732,12 +777,16 @@ __global__ void __launch_bounds__(kTriThreads, 2) quad_triangle_kernel(int t_lo,
 #pragma unroll
           for (int j = 0; j < 16; j += 2)
             if (j < nb) *reinterpret_cast<double2 *>(x + j) = make_double2(v[j], v[j + 1]);
-          S.phys[pos] = row;
           if (pos < c0 + nb) {
+            S.fin[pos] = row;
 #pragma unroll
             for (int j = 0; j < 16; ++j) S.l11[j][pos - c0] = v[j];
+          } else {
+            S.phys[par ^ 1][pos] = row;
           }
         }
+      } else if (c0 > 0) {
+        update(c0 - 16, S.phys[par], c0 + 16, kQuadRhsCol + 1, kTriPW);
       }
       __syncthreads();
       // U12 = L11^-1 A12, a column per thread (the right-hand side the last)
@@ -746,7 +795,7 @@ __global__ void __launch_bounds__(kTriThreads, 2) quad_triangle_kernel(int t_lo,
         double u[16];
         double *xc = X + cs + tid;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) u[i] = i < nb ? xc[S.phys[min(c0 + i, kQuadDim - 1)] * kTriS] : 0.0;
+        for (int i = 0; i < 16; ++i) u[i] = i < nb ? xc[S.fin[min(c0 + i, kQuadDim - 1)] * kTriS] : 0.0;
 #pragma unroll
         for (int i = 0; i < 15; ++i) {
           if (i >= nb) break;
@@ -756,43 +805,15 @@ __global__ void __launch_bounds__(kTriThreads, 2) quad_triangle_kernel(int t_lo,
         }
 #pragma unroll
         for (int i = 1; i < 16; ++i)
-          if (i < nb) xc[S.phys[min(c0 + i, kQuadDim - 1)] * kTriS] = u[i];
+          if (i < nb) xc[S.fin[min(c0 + i, kQuadDim - 1)] * kTriS] = u[i];
       }
       __syncthreads();
-      // A22 -= L21 U12 (panels before the last have 16 columns)
-      const int g = lane >> 2, t = lane & 3;
-      const int m2 = kQuadDim - cs, rts = (m2 + 15) / 16, cts = (m2 + 1 + 15) / 16;
-      for (int it2 = warp; m2 > 0 && it2 < rts * cts; it2 += kTriWarps) {
-        const int rt = it2 % rts, c = cs + 16 * (it2 / rts);
-        const int p0 = 16 * rt + g, p1 = p0 + 8;
-        double *x0 = X + S.phys[cs + min(p0, m2 - 1)] * kTriS, *x1 = X + S.phys[cs + min(p1, m2 - 1)] * kTriS;
-        double af[8], bf[2][4];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) af[q] = -((q & 1) ? x1 : x0)[c0 + t + 4 * (q >> 1)];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const double *u = X + S.phys[c0 + t + 4 * j] * kTriS;
-#pragma unroll
-          for (int ni = 0; ni < 2; ++ni) bf[ni][j] = u[min(c + 8 * ni + g, kQuadRhsCol)];
-        }
-#pragma unroll
-        for (int ni = 0; ni < 2; ++ni) {
-          const int cc = c + 8 * ni + 2 * t;  // this lane's two columns (the second may be the padding)
-          const bool cv = cc <= kQuadRhsCol;
-          double2 o0 = make_double2(0.0, 0.0), o1 = o0;
-          if (cv) {
-            o0 = *reinterpret_cast<const double2 *>(x0 + cc);
-            o1 = *reinterpret_cast<const double2 *>(x1 + cc);
-          }
-          double dd[4] = {o0.x, o0.y, o1.x, o1.y};
-          mma_f64_16816(dd, af, bf[ni]);
-          if (cv) {
-            if (p0 < m2) *reinterpret_cast<double2 *>(x0 + cc) = make_double2(dd[0], dd[1]);
-            if (p1 < m2) *reinterpret_cast<double2 *>(x1 + cc) = make_double2(dd[2], dd[3]);
-          }
-        }
+      // A22 -= L21 U12 on the next panel's columns, all warps (the last
+      // panel's columns are 112-115 and come with the right-hand side)
+      if (cs < kQuadDim) {
+        update(c0, S.phys[par ^ 1], cs, cs + 16 < kQuadDim ? cs + 16 : kQuadRhsCol + 1, 0);
+        __syncthreads();
       }
-      __syncthreads();
     }
     // back substitution by blocks of 16: the warp that holds the block's
     // positions solves its triangle, then every earlier position takes the
@@ -800,21 +821,21 @@ __global__ void __launch_bounds__(kTriThreads, 2) quad_triangle_kernel(int t_lo,
     if (warp < kTriPW) {
       double *xs = &S.c[0][0];
       const int k = tid;
-      const double *u = X + S.phys[min(k, kQuadDim - 1)] * kTriS;
-      double y = k < kQuadDim ? u[kQuadRhsCol] : 0.0;
-      const double d = k < kQuadDim ? u[k] : 1.0, rd = 1.0 / d;
+      const double *u = X + S.fin[min(k, kQuadDim - 1)] * kTriS;
+      // the row over its diagonal entry, so that the chain of unknowns is one
+      // product and one exchange each
+      const double rd = k < kQuadDim ? 1.0 / u[k] : 1.0;
+      double y = k < kQuadDim ? u[kQuadRhsCol] * rd : 0.0;
       for (int c0 = (kQuadDim - 1) / 16 * 16; c0 >= 0; c0 -= 16) {
         const int nb = min(16, kQuadDim - c0);
         if (warp == c0 / 32) {
-          for (int j = nb - 1; j >= 0; --j) {
-            const double q = y * rd;  // y / d with one residual correction (Markstein)
-            const double x = __shfl_sync(0xffffffffu, fma(fma(-q, d, y), rd, q), (c0 + j) & 31);
-            if (k == c0 + j) {
-              xs[k] = x;
-            } else if (k >= c0 && k < c0 + j) {
-              y = fma(-u[c0 + j], x, y);
-            }
-          }
+          double us[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) us[j] = (j < nb && k >= c0 && k < c0 + j) ? -u[c0 + j] * rd : 0.0;
+#pragma unroll
+          for (int j = 15; j >= 0; --j)
+            if (j < nb) y = fma(us[j], __shfl_sync(0xffffffffu, y, (c0 + j) & 31), y);
+          if (k >= c0 && k < c0 + nb) xs[k] = y;
         }
         asm volatile("bar.sync 1, %0;" ::"n"(32 * kTriPW) : "memory");
         if (k < c0) {
@@ -827,7 +848,7 @@ __global__ void __launch_bounds__(kTriThreads, 2) quad_triangle_kernel(int t_lo,
               s1 = fma(a.y, xs[c0 + j + 1], s1);
             }
           }
-          y -= s0 + s1;
+          y = fma(-rd, s0 + s1, y);
         }
       }
       if (tid < kQuadNbr) {
