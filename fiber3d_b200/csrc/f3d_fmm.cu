@@ -31,7 +31,7 @@
 //     m16n8k16).
 //   * Near field (the 27 neighbour leaves, both kernels, coincident points
 //     excluded) and the local expansion's evaluation at the targets (L2P)
-//     run in one kernel per target leaf.
+//     run in one kernel, at most 128 targets of a leaf per CTA.
 //   * Tree: Morton keys at depth 8, a bitonic sort of (key, index) pairs
 //     (deterministic), dense per-level slot tables built by a scan, the
 //     depth chosen as the smallest with at most max_pts sources per
@@ -344,14 +344,17 @@ __global__ void gather_kernel(const double *__restrict__ in, const uint64_t *__r
   out[e] = in[static_cast<int64_t>(src) * c + (e - i * c)];
 }
 
-// out[index of sorted element i] = scale * in[i] (3 values per point)
-__global__ void scatter_kernel(const double *__restrict__ in, const uint64_t *__restrict__ kv, int64_t n,
+// out[index of sorted element i] = scale * (the sum over splits of in[split][i],
+// in order; 3 values per point)
+__global__ void scatter_kernel(const double *__restrict__ in, int nsplit, const uint64_t *__restrict__ kv, int64_t n,
                                double scale, double *out) {
   const int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (e >= 3 * n) return;
   const int64_t i = e / 3;
   const uint32_t dst = static_cast<uint32_t>(kv[i]);
-  out[3 * static_cast<int64_t>(dst) + (e - 3 * i)] = scale * in[e];
+  double v = in[e];
+  for (int z = 1; z < nsplit; ++z) v += in[3 * n * z + e];
+  out[3 * static_cast<int64_t>(dst) + (e - 3 * i)] = scale * v;
 }
 
 // per-block min and max of three point sets (6 values per block)
@@ -406,7 +409,8 @@ __device__ __forceinline__ void box_center(const Geometry &g, int key, int level
 
 struct SourceSet {
   const double *xsl, *fsl;  // single layer: positions, forces (n x 3), sorted
-  const double *xdl, *ddl;  // double layer: positions (n x 3), tensors D (n x 9), sorted
+  const double *xdl, *ddl;  // double layer: positions (n x 3), tensors D (n x 9; null: D = 2 n (x) d), sorted
+  const double *ndl, *qdl;  // normals and densities (n x 3) where there are no tensors
   const int64_t *sl_start, *sl_end, *dl_start, *dl_end;  // per source leaf
 };
 
@@ -432,8 +436,6 @@ __global__ void __launch_bounds__(128) p2m_check_kernel(const Geometry g, int le
     const int64_t j0 = type == 0 ? src.sl_start[leaf] : src.dl_start[leaf];
     const int64_t j1 = type == 0 ? src.sl_end[leaf] : src.dl_end[leaf];
     const double *px = type == 0 ? src.xsl : src.xdl;
-    const double *pv = type == 0 ? src.fsl : src.ddl;
-    const int nv = type == 0 ? 3 : 9;
     for (int64_t jb = j0; jb < j1; jb += 128) {
       const int cnt = static_cast<int>(min(static_cast<int64_t>(128), j1 - jb));
       __syncthreads();
@@ -441,7 +443,14 @@ __global__ void __launch_bounds__(128) p2m_check_kernel(const Geometry g, int le
         const int64_t j = jb + threadIdx.x;
 #pragma unroll
         for (int d = 0; d < 3; ++d) sp[threadIdx.x][d] = px[3 * j + d];
-        for (int q = 0; q < nv; ++q) sv[threadIdx.x][q] = pv[nv * j + q];
+        if (type == 0) {
+          for (int q = 0; q < 3; ++q) sv[threadIdx.x][q] = src.fsl[3 * j + q];
+        } else if (src.ddl) {
+          for (int q = 0; q < 9; ++q) sv[threadIdx.x][q] = src.ddl[9 * j + q];
+        } else {  // D = 2 n (x) d (fiber3d's convention for STKFMM, kernels.py:1410)
+#pragma unroll
+          for (int q = 0; q < 9; ++q) sv[threadIdx.x][q] = 2.0 * src.ndl[3 * j + q / 3] * src.qdl[3 * j + q % 3];
+        }
       }
       __syncthreads();
       if (!kv) continue;
@@ -742,6 +751,11 @@ __global__ void split_sum_kernel(const double *__restrict__ partial, int nsplit,
 
 
 // ------------------------------------------------------------ near field + L2P --
+constexpr int kNearThreads = 64;
+constexpr int kNearTargets = 2 * kNearThreads;  // of one item: two per thread
+constexpr int kNearStages = 3;
+constexpr int kNearMaxSplit = 9;
+
 struct NearArgs {
   Geometry g;
   int level;
@@ -753,118 +767,219 @@ struct NearArgs {
   const double *psi;                    // downward equivalent densities (4n per target leaf)
   const double *surf;
   int n;
-  double *out;                          // sorted targets x 3
+  const int *item_off;                  // first item of each target leaf (one per kNearTargets targets)
+  const int *item_leaf;                 // leaf of each item
+  int64_t ntrg;
+  double *out;                          // [splits][sorted targets][3]
 };
 
-// Two targets per thread (t and t + 128 of a 256-target block of the leaf):
-// each staged source serves both.
-__global__ void __launch_bounds__(128) near_l2p_kernel(const NearArgs a) {
-  __shared__ double sp[128][3], sv[128][9];
-  const int leaf = blockIdx.x;
+// items of each target leaf
+__global__ void near_count_kernel(const int64_t *__restrict__ start, const int64_t *__restrict__ end, int nleaf,
+                                  int *count) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < nleaf) count[i] = static_cast<int>((end[i] - start[i] + kNearTargets - 1) / kNearTargets);
+}
+
+// leaf of each item from the items' offsets
+__global__ void near_items_kernel(const int *__restrict__ off, int nleaf, int nitems, int *leaf) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nleaf) return;
+  const int e = i + 1 < nleaf ? off[i + 1] : nitems;
+  for (int k = off[i]; k < e; ++k) leaf[k] = i;
+}
+
+__device__ __forceinline__ void cp_async8(double *smem, const double *gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(smem)), "l"(gmem) : "memory");
+}
+
+// The near field (27 neighbour leaves, both layers; pairs closer than 1e-150
+// excluded, as STKFMM's kernels exclude coincident points) and the leaf's
+// local expansion at the targets.
+//
+// Bound by the FP64 pipe (25 instructions a pair) once the GPU is evenly
+// filled, which whole leaves do not do: at 1e5 points of each kind some 340
+// of 512 leaves hold nearly all targets.  So an item is at most 128 targets
+// of a leaf (64 threads, two targets each), the 27 leaves are split over
+// gridDim.y where the items are few (partial sums, added in order by the
+// scatter), and the sources of an item's leaves run as one list through a
+// three-stage ring of 64 (cp.async), so that only its last tile is ragged.
+// Double-layer sources given as normal and density take (n.r)(d.r), 7
+// instructions, instead of the tensor's r^T D r, 12; the exclusion of
+// coincident points compares bits on the integer pipe.  One evaluation's near
+// field: 2.93 ms at 1e5 points of each kind (8.4 ms for a CTA of 128 threads
+// per leaf), 38.4 ms at 1e6 (48.3 ms).
+template <bool TENSOR>
+__global__ void __launch_bounds__(kNearThreads) near_l2p_kernel(const NearArgs a) {
+  constexpr int kRec = TENSOR ? 12 : 10;  // doubles per staged source
+  __shared__ __align__(16) double st[kNearStages][kNearThreads][kRec];
+  __shared__ int64_t s_start[2][27];
+  __shared__ int s_pref[2][28];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int leaf = a.item_leaf[blockIdx.x];
   const int key = a.trg_keys[leaf];
   double c[3], h;
   box_center(a.g, key, a.level, c, h);
-  int bx, by, bz;
-  unmorton(static_cast<uint32_t>(key), bx, by, bz);
-  const int m = 1 << a.level;
-  const int64_t t0 = a.trg_start[leaf], t1 = a.trg_end[leaf];
-  for (int64_t tb = t0; tb < t1; tb += 256) {
-    double x[2][3];
-    bool iv[2];
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int64_t i = tb + threadIdx.x + 128 * q;
-      iv[q] = i < t1;
-#pragma unroll
-      for (int d = 0; d < 3; ++d) x[q][d] = iv[q] ? a.xt[3 * i + d] : c[d];
+  const int64_t t0 = a.trg_start[leaf] + static_cast<int64_t>(static_cast<int>(blockIdx.x) - a.item_off[leaf]) * kNearTargets;
+  const int64_t t1 = a.trg_end[leaf];
+  {  // warp w: this split's leaves of layer w as one list
+    int64_t start = 0;
+    int cnt = 0;
+    if (lane >= static_cast<int>(27 * blockIdx.y / gridDim.y) && lane < static_cast<int>(27 * (blockIdx.y + 1) / gridDim.y)) {
+      int bx, by, bz;
+      unmorton(static_cast<uint32_t>(key), bx, by, bz);
+      const int m = 1 << a.level;
+      const int nx = bx + lane / 9 - 1, ny = by + (lane / 3) % 3 - 1, nz = bz + lane % 3 - 1;
+      if (nx >= 0 && ny >= 0 && nz >= 0 && nx < m && ny < m && nz < m) {
+        const int slot = a.src_table[morton(nx, ny, nz)];
+        if (slot >= 0) {
+          start = warp ? a.src.dl_start[slot] : a.src.sl_start[slot];
+          cnt = static_cast<int>((warp ? a.src.dl_end[slot] : a.src.sl_end[slot]) - start);
+        }
+      }
     }
-    double us[2][3] = {}, ud[2][3] = {}, uf[2][3] = {};
-    for (int nb = 0; nb < 27; ++nb) {
-      const int nx = bx + nb / 9 - 1, ny = by + (nb / 3) % 3 - 1, nz = bz + nb % 3 - 1;
-      if (nx < 0 || ny < 0 || nz < 0 || nx >= m || ny >= m || nz >= m) continue;
-      const int slot = a.src_table[morton(nx, ny, nz)];
-      if (slot < 0) continue;
-      // single layer
-      for (int64_t jb = a.src.sl_start[slot], j1 = a.src.sl_end[slot]; jb < j1; jb += 128) {
-        const int cnt = static_cast<int>(min(static_cast<int64_t>(128), j1 - jb));
-        __syncthreads();
-        if (threadIdx.x < cnt) {
-          const int64_t j = jb + threadIdx.x;
+    const int incl = warp_incl_scan(cnt);
+    if (lane < 27) {
+      s_start[warp][lane] = start;
+      s_pref[warp][lane + 1] = incl;
+    }
+    if (lane == 0) s_pref[warp][0] = 0;
+  }
+  double x[2][3];
+  bool iv[2];
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const int64_t i = t0 + tid + kNearThreads * q;
+    iv[q] = i < t1;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) x[q][d] = iv[q] ? a.xt[3 * i + d] : c[d];
+  }
+  __syncthreads();
+
+  // sources total of layer w, 64 at a time: `copy(dst, j)` requests source j,
+  // `term(record)` adds one staged source
+  auto sweep = [&](int w, auto copy, auto term) {
+    const int total = s_pref[w][27], tiles = (total + kNearThreads - 1) / kNearThreads;
+    int b = 0;  // this thread's source's leaf (its sources only move forward)
+    auto load = [&](int tile) {
+      const int k = tile * kNearThreads + tid;
+      if (k < total) {
+        while (s_pref[w][b + 1] <= k) ++b;
+        copy(st[tile % kNearStages][tid], s_start[w][b] + (k - s_pref[w][b]));
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    load(0);
+    load(1);
+    for (int tile = 0; tile < tiles; ++tile) {
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+      __syncthreads();
+      load(tile + 2);  // into the stage of tile - 1, which every thread has left
+      const int cnt = min(kNearThreads, total - tile * kNearThreads);
+      const double(*rec)[kRec] = st[tile % kNearStages];
+#pragma unroll 2
+      for (int s = 0; s < cnt; ++s) term(rec[s]);
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+  };
+  const long long tiny = __double_as_longlong(kCoincident2);
+  double us[2][3] = {}, ud[2][3] = {}, uf[2][3] = {};
+  sweep(
+      0,
+      [&](double *dst, int64_t j) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          cp_async8(dst + d, a.src.xsl + 3 * j + d);
+          cp_async8(dst + 3 + d, a.src.fsl + 3 * j + d);
+        }
+      },
+      [&](const double *r) {
+        const double2 u0 = *reinterpret_cast<const double2 *>(r), u1 = *reinterpret_cast<const double2 *>(r + 2),
+                      u2 = *reinterpret_cast<const double2 *>(r + 4);
+        const double f0 = u1.y, f1 = u2.x, f2 = u2.y;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const double r0 = x[q][0] - u0.x, r1 = x[q][1] - u0.y, r2 = x[q][2] - u1.x;
+          const double d2 = fma(r0, r0, fma(r1, r1, r2 * r2));
+          double ri = rsqrt_refined(d2);
+          ri = __double_as_longlong(d2) > tiny ? ri : 0.0;
+          const double g3 = ri * ri * ri * fma(r0, f0, fma(r1, f1, r2 * f2));
+          us[q][0] = fma(g3, r0, fma(ri, f0, us[q][0]));
+          us[q][1] = fma(g3, r1, fma(ri, f1, us[q][1]));
+          us[q][2] = fma(g3, r2, fma(ri, f2, us[q][2]));
+        }
+      });
+  sweep(
+      1,
+      [&](double *dst, int64_t j) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) cp_async8(dst + d, a.src.xdl + 3 * j + d);
+        if (TENSOR) {
+#pragma unroll
+          for (int e = 0; e < 9; ++e) cp_async8(dst + 3 + e, a.src.ddl + 9 * j + e);
+        } else {
 #pragma unroll
           for (int d = 0; d < 3; ++d) {
-            sp[threadIdx.x][d] = a.src.xsl[3 * j + d];
-            sv[threadIdx.x][d] = a.src.fsl[3 * j + d];
+            cp_async8(dst + 3 + d, a.src.ndl + 3 * j + d);
+            cp_async8(dst + 6 + d, a.src.qdl + 3 * j + d);
           }
         }
-        __syncthreads();
-        for (int s = 0; s < cnt; ++s) {
-          const double p0 = sp[s][0], p1 = sp[s][1], p2 = sp[s][2];
-          const double f0 = sv[s][0], f1 = sv[s][1], f2 = sv[s][2];
+      },
+      [&](const double *r) {
+        double v[kRec];
 #pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            const double r0 = x[q][0] - p0, r1 = x[q][1] - p1, r2 = x[q][2] - p2;
-            const double d2 = fma(r0, r0, fma(r1, r1, r2 * r2));
-            double ri = rsqrt_refined(d2);
-            ri = d2 > kCoincident2 ? ri : 0.0;
-            const double g3 = ri * ri * ri * fma(r0, f0, fma(r1, f1, r2 * f2));
-            us[q][0] = fma(g3, r0, fma(ri, f0, us[q][0]));
-            us[q][1] = fma(g3, r1, fma(ri, f1, us[q][1]));
-            us[q][2] = fma(g3, r2, fma(ri, f2, us[q][2]));
+        for (int e = 0; e < kRec; e += 2) {
+          if (!TENSOR && e == 8) {
+            v[8] = r[8];
+          } else {
+            const double2 u = *reinterpret_cast<const double2 *>(r + e);
+            v[e] = u.x;
+            v[e + 1] = u.y;
           }
         }
-      }
-      // double layer
-      for (int64_t jb = a.src.dl_start[slot], j1 = a.src.dl_end[slot]; jb < j1; jb += 128) {
-        const int cnt = static_cast<int>(min(static_cast<int64_t>(128), j1 - jb));
-        __syncthreads();
-        if (threadIdx.x < cnt) {
-          const int64_t j = jb + threadIdx.x;
 #pragma unroll
-          for (int d = 0; d < 3; ++d) sp[threadIdx.x][d] = a.src.xdl[3 * j + d];
-#pragma unroll
-          for (int e = 0; e < 9; ++e) sv[threadIdx.x][e] = a.src.ddl[9 * j + e];
-        }
-        __syncthreads();
-        for (int s = 0; s < cnt; ++s) {
-          const double p0 = sp[s][0], p1 = sp[s][1], p2 = sp[s][2];
-          const double *D = sv[s];
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            const double r0 = x[q][0] - p0, r1 = x[q][1] - p1, r2 = x[q][2] - p2;
-            const double d2 = fma(r0, r0, fma(r1, r1, r2 * r2));
-            const double qq = r0 * fma(D[0], r0, fma(D[1], r1, D[2] * r2)) +
-                              r1 * fma(D[3], r0, fma(D[4], r1, D[5] * r2)) +
-                              r2 * fma(D[6], r0, fma(D[7], r1, D[8] * r2));
-            double f = times_rsqrt5(qq, d2);
-            f = d2 > kCoincident2 ? f : 0.0;
-            ud[q][0] = fma(f, r0, ud[q][0]);
-            ud[q][1] = fma(f, r1, ud[q][1]);
-            ud[q][2] = fma(f, r2, ud[q][2]);
+        for (int q = 0; q < 2; ++q) {
+          const double r0 = x[q][0] - v[0], r1 = x[q][1] - v[1], r2 = x[q][2] - v[2];
+          const double d2 = fma(r0, r0, fma(r1, r1, r2 * r2));
+          double qq;
+          if (TENSOR) {
+            const double *D = v + 3;
+            qq = r0 * fma(D[0], r0, fma(D[1], r1, D[2] * r2)) + r1 * fma(D[3], r0, fma(D[4], r1, D[5] * r2)) +
+                 r2 * fma(D[6], r0, fma(D[7], r1, D[8] * r2));
+          } else {
+            qq = fma(v[3], r0, fma(v[4], r1, v[5] * r2)) * fma(v[6], r0, fma(v[7], r1, v[8] * r2));
           }
+          double f = times_rsqrt5(qq, d2);
+          f = __double_as_longlong(d2) > tiny ? f : 0.0;
+          ud[q][0] = fma(f, r0, ud[q][0]);
+          ud[q][1] = fma(f, r1, ud[q][1]);
+          ud[q][2] = fma(f, r2, ud[q][2]);
         }
-      }
-    }
-    // the local expansion: K4 from the leaf's downward equivalent surface,
-    // source component q scaled back by h
+      });
+  // the local expansion (first split): K4 from the leaf's downward equivalent
+  // surface, source component q scaled back by h
+  if (blockIdx.y == 0) {
     const double *psi = a.psi + static_cast<int64_t>(leaf) * 4 * a.n;
-    for (int kb = 0; kb < a.n; kb += 128) {
-      const int cnt = min(128, a.n - kb);
-      __syncthreads();
-      if (threadIdx.x < cnt) {
-        const int k = kb + threadIdx.x;
+    for (int kb = 0; kb < a.n; kb += kNearThreads) {
+      const int cnt = min(kNearThreads, a.n - kb);
+      if (tid < cnt) {
+        const int k = kb + tid;
+        double *dst = st[0][tid];
 #pragma unroll
-        for (int d = 0; d < 3; ++d) sp[threadIdx.x][d] = c[d] + kRout * h * a.surf[3 * k + d];
+        for (int d = 0; d < 3; ++d) dst[d] = c[d] + kRout * h * a.surf[3 * k + d];
 #pragma unroll
-        for (int e = 0; e < 3; ++e) sv[threadIdx.x][e] = psi[4 * k + e];
-        sv[threadIdx.x][3] = h * psi[4 * k + 3];
+        for (int e = 0; e < 3; ++e) dst[3 + e] = psi[4 * k + e];
+        dst[6] = h * psi[4 * k + 3];
       }
       __syncthreads();
       for (int s = 0; s < cnt; ++s) {
-        const double p0 = sp[s][0], p1 = sp[s][1], p2 = sp[s][2];
-        const double f0 = sv[s][0], f1 = sv[s][1], f2 = sv[s][2], fq = sv[s][3];
+        const double *r = st[0][s];
+        const double2 u0 = *reinterpret_cast<const double2 *>(r), u1 = *reinterpret_cast<const double2 *>(r + 2),
+                      u2 = *reinterpret_cast<const double2 *>(r + 4);
+        const double f0 = u1.y, f1 = u2.x, f2 = u2.y, fq = r[6];
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-          const double r0 = x[q][0] - p0, r1 = x[q][1] - p1, r2 = x[q][2] - p2;
+          const double r0 = x[q][0] - u0.x, r1 = x[q][1] - u0.y, r2 = x[q][2] - u1.x;
           const double ri = rsqrt_refined(fma(r0, r0, fma(r1, r1, r2 * r2)));
           const double g3 = ri * ri * ri * (fma(r0, f0, fma(r1, f1, r2 * f2)) + fq);
           uf[q][0] = fma(g3, r0, fma(ri, f0, uf[q][0]));
@@ -872,27 +987,18 @@ __global__ void __launch_bounds__(128) near_l2p_kernel(const NearArgs a) {
           uf[q][2] = fma(g3, r2, fma(ri, f2, uf[q][2]));
         }
       }
-    }
-    const double cs = 1.0 / (8.0 * kPi), cd = -3.0 / (8.0 * kPi);
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      if (!iv[q]) continue;
-      const int64_t i = tb + threadIdx.x + 128 * q;
-#pragma unroll
-      for (int d = 0; d < 3; ++d) a.out[3 * i + d] = fma(cs, us[q][d], fma(cd, ud[q][d], uf[q][d]));
+      __syncthreads();
     }
   }
-}
-
-// D = 2 n (x) d per double-layer source (fiber3d's convention for STKFMM,
-// kernels.py:1410)
-__global__ void dl_tensor_kernel(const double *__restrict__ nrm, const double *__restrict__ dens, int64_t n,
-                                 double *D) {
-  const int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (e >= 9 * n) return;
-  const int64_t i = e / 9;
-  const int jk = static_cast<int>(e - 9 * i);
-  D[e] = 2.0 * nrm[3 * i + jk / 3] * dens[3 * i + jk % 3];
+  // D = 2 n (x) d: the factor 2 of the normal-and-density form goes here
+  const double cs = 1.0 / (8.0 * kPi), cd = (TENSOR ? -3.0 : -6.0) / (8.0 * kPi);
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    if (!iv[q]) continue;
+    double *o = a.out + 3 * (blockIdx.y * a.ntrg + t0 + tid + kNearThreads * q);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) o[d] = fma(cs, us[q][d], fma(cd, ud[q][d], uf[q][d]));
+  }
 }
 
 }  // namespace fmm
@@ -950,7 +1056,9 @@ struct f3d_fmm {
   int depth = 0;
   DevBuf kv_sl, kv_dl, kv_trg;          // sorted (key << 32 | index), padded
   DevBuf x_sl, x_dl, x_trg;             // sorted coordinates
-  DevBuf f_sl, d_dl, dl_tmp;            // sorted densities (3 and 9 per point)
+  DevBuf f_sl, d_dl;                    // sorted densities (3 per point; 9, or normal and density 3 + 3)
+  DevBuf item_off, item_leaf;           // near-field items of each target leaf, leaf of each item
+  int nitems = 0;
   DevBuf sl_start, sl_end, dl_start, dl_end, trg_start, trg_end;
   DevBuf flags, tile_sums, scalars, okv, ybuf, out_sorted, bbox, split_partial;
   int64_t m2l_pairs = 0;  // non-empty interaction-list entries over all levels
@@ -1055,6 +1163,19 @@ int build_tree(f3d_fmm *h, cudaStream_t st) {
   leaf_ranges_kernel<<<blocks(h->ntrg), 256, 0, st>>>(as<uint64_t>(h->kv_trg), h->ntrg, shift, as<int>(leaf.trg_table),
                                                       as<int64_t>(h->trg_start), as<int64_t>(h->trg_end));
   if ((rc = launch_status())) return rc;
+  // near-field items: at most kNearTargets targets of one leaf each
+  {
+    if ((rc = reserve(h->item_off, static_cast<size_t>(leaf.ntrg) * sizeof(int)))) return rc;
+    near_count_kernel<<<blocks(leaf.ntrg), 256, 0, st>>>(as<int64_t>(h->trg_start), as<int64_t>(h->trg_end), leaf.ntrg,
+                                                         as<int>(h->item_off));
+    if ((rc = launch_status())) return rc;
+    if ((rc = scan_exclusive(as<int>(h->item_off), leaf.ntrg, as<int>(h->tile_sums), as<int>(h->scalars), st))) return rc;
+    if ((rc = sync_read(&h->nitems, h->scalars.p, sizeof(int), st))) return rc;
+    if ((rc = reserve(h->item_leaf, static_cast<size_t>(h->nitems) * sizeof(int)))) return rc;
+    near_items_kernel<<<blocks(leaf.ntrg), 256, 0, st>>>(as<int>(h->item_off), leaf.ntrg, h->nitems,
+                                                         as<int>(h->item_leaf));
+    if ((rc = launch_status())) return rc;
+  }
   // upper levels: parents of the boxes below
   for (int l = L - 1; l >= 2; --l) {
     const int64_t nk = int64_t(1) << (3 * l);
@@ -1220,7 +1341,7 @@ int f3d_fmm_destroy(f3d_fmm *h) {
     b.p = nullptr;
   };
   for (DevBuf *b : {&h->surf, &h->uc2ue, &h->dc2de, &h->kv_sl, &h->kv_dl, &h->kv_trg, &h->x_sl, &h->x_dl, &h->x_trg,
-                    &h->f_sl, &h->d_dl, &h->dl_tmp, &h->sl_start, &h->sl_end, &h->dl_start, &h->dl_end,
+                    &h->f_sl, &h->d_dl, &h->item_off, &h->item_leaf, &h->sl_start, &h->sl_end, &h->dl_start, &h->dl_end,
                     &h->trg_start, &h->trg_end, &h->flags, &h->tile_sums, &h->scalars, &h->okv, &h->ybuf,
                     &h->out_sorted, &h->bbox, &h->split_partial})
     release(*b);
@@ -1312,33 +1433,37 @@ int f3d_fmm_evaluate(f3d_fmm *h, const double *sl_density, const double *dl_norm
   if (h->depth < 2) return F3D_ERR_ARG;  // set_points has not run for these points
   int rc;
   const int n = h->n, n3 = 3 * n, n4 = 4 * n, L = h->depth;
+  // The near field's 27 leaves are split where its items (128 targets each)
+  // are fewer than 32 per SM: about three resident sets of ten, so that the
+  // last one is a small part of the whole.
+  const int nsplit = std::max(1, std::min(kNearMaxSplit, 32 * sm_count() / std::max(1, h->nitems)));
   // densities in sorted order
   if ((rc = reserve(h->f_sl, std::max<size_t>(nsl, 1) * 3 * sizeof(double))) ||
-      (rc = reserve(h->d_dl, std::max<size_t>(ndl, 1) * 9 * sizeof(double))) ||
-      (rc = reserve(h->out_sorted, static_cast<size_t>(ntrg) * 3 * sizeof(double))))
+      (rc = reserve(h->d_dl, std::max<size_t>(ndl, 1) * (dl_tensor ? 9 : 6) * sizeof(double))) ||
+      (rc = reserve(h->out_sorted, static_cast<size_t>(nsplit) * ntrg * 3 * sizeof(double))))
     return rc;
   h->launches = 0;
   if (nsl) {
     gather_kernel<<<blocks(3 * nsl), 256, 0, st>>>(sl_density, as<uint64_t>(h->kv_sl), nsl, 3, as<double>(h->f_sl));
     ++h->launches;
   }
-  if (ndl) {
-    const double *D = dl_tensor;
-    if (!D) {
-      if ((rc = reserve(h->dl_tmp, static_cast<size_t>(ndl) * 9 * sizeof(double)))) return rc;
-      dl_tensor_kernel<<<blocks(9 * ndl), 256, 0, st>>>(dl_normal, dl_density, ndl, as<double>(h->dl_tmp));
-      ++h->launches;
-      D = as<double>(h->dl_tmp);
-    }
-    gather_kernel<<<blocks(9 * ndl), 256, 0, st>>>(D, as<uint64_t>(h->kv_dl), ndl, 9, as<double>(h->d_dl));
+  if (ndl && dl_tensor) {
+    gather_kernel<<<blocks(9 * ndl), 256, 0, st>>>(dl_tensor, as<uint64_t>(h->kv_dl), ndl, 9, as<double>(h->d_dl));
     ++h->launches;
+  } else if (ndl) {
+    gather_kernel<<<blocks(3 * ndl), 256, 0, st>>>(dl_normal, as<uint64_t>(h->kv_dl), ndl, 3, as<double>(h->d_dl));
+    gather_kernel<<<blocks(3 * ndl), 256, 0, st>>>(dl_density, as<uint64_t>(h->kv_dl), ndl, 3,
+                                                   as<double>(h->d_dl) + 3 * ndl);
+    h->launches += 2;
   }
   if ((rc = launch_status())) return rc;
   SourceSet src{};
   src.xsl = as<double>(h->x_sl);
   src.fsl = as<double>(h->f_sl);
   src.xdl = as<double>(h->x_dl);
-  src.ddl = as<double>(h->d_dl);
+  src.ddl = dl_tensor ? as<double>(h->d_dl) : nullptr;
+  src.ndl = as<double>(h->d_dl);
+  src.qdl = as<double>(h->d_dl) + 3 * ndl;
   src.sl_start = as<int64_t>(h->sl_start);
   src.sl_end = as<int64_t>(h->sl_end);
   src.dl_start = as<int64_t>(h->dl_start);
@@ -1460,10 +1585,17 @@ int f3d_fmm_evaluate(f3d_fmm *h, const double *sl_density, const double *dl_norm
   na.psi = as<double>(leaf.psi);
   na.surf = surf;
   na.n = n;
+  na.item_off = as<int>(h->item_off);
+  na.item_leaf = as<int>(h->item_leaf);
+  na.ntrg = ntrg;
   na.out = as<double>(h->out_sorted);
-  near_l2p_kernel<<<static_cast<unsigned>(leaf.ntrg), 128, 0, st>>>(na);
+  const dim3 ngrid(static_cast<unsigned>(h->nitems), static_cast<unsigned>(nsplit));
+  if (dl_tensor)
+    near_l2p_kernel<true><<<ngrid, kNearThreads, 0, st>>>(na);
+  else
+    near_l2p_kernel<false><<<ngrid, kNearThreads, 0, st>>>(na);
   h->launches += 2;  // with the scatter below
-  scatter_kernel<<<blocks(3 * ntrg), 256, 0, st>>>(as<double>(h->out_sorted), as<uint64_t>(h->kv_trg), ntrg,
+  scatter_kernel<<<blocks(3 * ntrg), 256, 0, st>>>(as<double>(h->out_sorted), nsplit, as<uint64_t>(h->kv_trg), ntrg,
                                                    1.0 / eta, out);
   return launch_status();
 }
