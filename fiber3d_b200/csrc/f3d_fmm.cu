@@ -293,7 +293,11 @@ __global__ void leaf_ranges_kernel(const uint64_t *__restrict__ kv, int64_t n, i
   if (i == n - 1 || (static_cast<uint32_t>(kv[i + 1] >> 32) >> shift) != k) end[slot] = i + 1;
 }
 
-// (octant << 32 | slot) of every box of a level, for grouping by octant
+// (octant, coordinates, slot) of every box of a level, for grouping by octant;
+// coordinate order within one, so that runs of eight columns near a face of the
+// domain lack the same terms of the interaction list (18 % of the products left
+// out at 8^3 and 17 % at 16^3 leaves; grouping by faces first leaves out 27 % and
+// 23 % but no time: the warps of a tile wait for the one with the most)
 __global__ void octant_keys_kernel(const int *__restrict__ keys, int nbox, int64_t n2, uint64_t *kv,
                                    unsigned *oct_count) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -303,7 +307,10 @@ __global__ void octant_keys_kernel(const int *__restrict__ keys, int nbox, int64
     return;
   }
   const unsigned oct = static_cast<unsigned>(keys[i]) & 7u;
-  kv[i] = (static_cast<uint64_t>(oct) << 32) | static_cast<uint32_t>(i);
+  int ix, iy, iz;
+  unmorton(static_cast<uint32_t>(keys[i]), ix, iy, iz);
+  const uint64_t at = static_cast<uint64_t>((ix << 16) | (iy << 8) | iz);
+  kv[i] = (static_cast<uint64_t>(oct) << 56) | (at << 32) | static_cast<uint32_t>(i);
   atomicAdd(&oct_count[oct], 1u);
 }
 
@@ -497,7 +504,8 @@ __global__ void __launch_bounds__(128) p2m_check_kernel(const Geometry g, int le
 // The columns of M2L are grouped by octant; a CTA's 64 columns share one.
 // Terms are split over grid.z; each split writes its own partial and a
 // second kernel adds the partials in split order (deterministic).
-constexpr int GBM = 96, GBN = 64, GBK = 32, GTHREADS = 128;
+constexpr int GBM = 48, GBN = 64, GBK = 32, GTHREADS = 128;
+constexpr int kSplitRows = 96;  // row tile behind the split count, which fixes the order of the sums
 // shared row strides (doubles), 4 mod 16: the tensor-core fragment reads of
 // a half-warp (A: k = t + 4q, row g; B: k = t + 4j, column g) hit 16
 // different bank pairs
@@ -533,6 +541,12 @@ struct GemmOp {
   const double *X, *X2;
   int ldx;
 };
+
+// 8 bytes to shared memory, or zeros
+__device__ __forceinline__ void cp_async8z(double *smem, const double *gmem, bool valid) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_addr(smem)), "l"(gmem), "r"(valid ? 8 : 0)
+               : "memory");
+}
 
 struct TermGeom {
   double off[3];
@@ -597,143 +611,225 @@ __device__ __forceinline__ int source_slot(const GemmOp &op, int oct, int slot, 
   return op.table[morton(ix, iy, iz)];
 }
 
-__global__ void __launch_bounds__(GTHREADS) fmm_gemm_kernel(const __grid_constant__ GemmOp op) {
-  __shared__ __align__(16) double As[GBK][GAS];
-  __shared__ __align__(16) double Xs[GBK][GXS];
-  __shared__ int s_src[GBN];
-  __shared__ int s_any;
+// The chunks (32 k) of all the terms of an item (48 rows x 64 columns of one
+// split) form one stream through two buffers: while chunk i is multiplied,
+// chunk i + 1's densities arrive by cp.async and its kernel values are formed,
+// with one barrier per chunk.  Groups of 8
+// columns without a source in a term (boxes near the domain's faces, kept
+// together) take no products.
+//
+// Bound by the FP64 tensor cores on an SM that has work; what decides is how
+// evenly the items fall on the SMs.  Items of 96 rows, a CTA each, left between
+// three and six on an SM at 1e5 points (640 CTAs, three resident: 10.3 ms, the
+// tensor pipe 81 % active on the busiest SM and 42 % on the idlest).  So items
+// are half as tall and a persistent grid takes them in turn, which puts eight
+// or nine on each.  Then the instructions around the products: 428 per warp and
+// 16 k with the gather's addresses formed for each value, 270 with a pointer per
+// column moved on; and 32 k per barrier instead of 16.  All launches of an
+// evaluation at 1e5 points of each kind, order 8: 12.7 ms before, 12.3 (even
+// items), 10.7 (pointers), 9.9 (32 k); at 1e6 70.0 before, 54.2 ms.  The order of
+// every sum is as it was: at order 8 the check-to-equivalent maps turn a
+// rounding there into 1e-8 of the result.
+__global__ void __launch_bounds__(GTHREADS, 3) fmm_gemm_kernel(const __grid_constant__ GemmOp op, int rtiles,
+                                                               int ctiles) {
+  extern __shared__ __align__(16) double g_smem[];
+  auto As = reinterpret_cast<double(*)[GBK][GAS]>(g_smem);                       // [2][GBK][GAS]
+  auto Xs = reinterpret_cast<double(*)[GBK][GXS]>(g_smem + 2 * GBK * GAS);       // [2][GBK][GXS]
+  __shared__ int s_src[2][GBN];        // source box of each column, by term parity
+  __shared__ unsigned s_live[2][2];    // its columns that have one
   const int tid = threadIdx.x;
-  const int row0 = blockIdx.x * GBM;
-  // the column tile's octant group
-  const int tile = blockIdx.y;
-  int oct = 0;
-  while (oct < 7 && tile >= op.oct_tile_start[oct + 1]) ++oct;
-  const int col0 = op.oct_col_start[oct] + (tile - op.oct_tile_start[oct]) * GBN;
-  const int col_end = op.oct_col_start[oct + 1];
   const int tps = (op.nterms + op.nsplit - 1) / op.nsplit;
-  const int t_lo = blockIdx.z * tps, t_hi = min(op.nterms, t_lo + tps);
-  // FP64 tensor cores (mma.sync m16n8k16): warp w computes rows
-  // 48 (w / 2) .. + 47 and columns 32 (w % 2) .. + 31 of the tile as 3 x 4
-  // tiles of 16 x 8; lane = 4 lg + t4 holds rows lg, lg + 8 and columns
-  // 2 t4, 2 t4 + 1 of each
+  // FP64 tensor cores (mma.sync m16n8k16): warp w computes columns 16 w .. + 15
+  // of the tile as 3 x 2 tiles of 16 x 8; lane = 4 lg + t4 holds rows lg,
+  // lg + 8 and columns 2 t4, 2 t4 + 1 of each
   const int lane = tid & 31, warp = tid >> 5;
   const int lg = lane >> 2, t4 = lane & 3;
-  const int wr = 48 * (warp >> 1), wc = 32 * (warp & 1);
-  double acc[3][4][4];
+  const int wc = 16 * warp;
+  // kernel values: one check point and one of a chunk's eight equivalent points per thread
+  const int gi = tid % (GBM / 3), ge = tid / (GBM / 3);
+  const int chunks = (op.K + GBK - 1) / GBK;
+  const int64_t items = static_cast<int64_t>(rtiles) * ctiles * op.nsplit;
+  for (int64_t item = blockIdx.x; item < items; item += gridDim.x) {
+    const int row0 = static_cast<int>(item % rtiles) * GBM;
+    const int tile = static_cast<int>(item / rtiles % ctiles), split = static_cast<int>(item / rtiles / ctiles);
+    // the column tile's octant group
+    int oct = 0;
+    while (oct < 7 && tile >= op.oct_tile_start[oct + 1]) ++oct;
+    const int col0 = op.oct_col_start[oct] + (tile - op.oct_tile_start[oct]) * GBN;
+    const int col_end = op.oct_col_start[oct + 1];
+    const int t_lo = split * tps, t_hi = min(op.nterms, t_lo + tps);
+    double acc[3][2][4];
 #pragma unroll
-  for (int mi = 0; mi < 3; ++mi)
+    for (int mi = 0; mi < 3; ++mi)
 #pragma unroll
-    for (int ni = 0; ni < 4; ++ni)
+      for (int ni = 0; ni < 2; ++ni)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) acc[mi][ni][i] = 0.0;
+        for (int i = 0; i < 4; ++i) acc[mi][ni][i] = 0.0;
 
-  for (int t = t_lo; t < t_hi; ++t) {
-    if (tid == 0) s_any = 0;
-    __syncthreads();
-    if (tid < GBN) {
-      const int col = col0 + tid;
-      int s = -1;
-      if (col < col_end) s = source_slot(op, oct, op.cols ? op.cols[col] : col, t);
-      s_src[tid] = s;
-      if (s >= 0) s_any = 1;
+    // the producer's place in the stream: chunk pk of term pt (the term's
+    // sources in s_src[pbuf]); this thread's four columns' densities at that
+    // chunk (their bit in pv set where the column has a source)
+    int pt = t_lo - 1, pk = 0, pbuf = 1;
+    const double *px[4];
+    unsigned pv = 0;
+    TermGeom pg{};
+    const double *pa = nullptr;  // GEN_STORED: this thread's entry of A in the chunk
+    double cs[3] = {0.0, 0.0, 0.0};  // this thread's check point
+    const bool gv = op.mode != GEN_STORED && row0 / 3 + gi < op.n;
+    if (gv) {
+#pragma unroll
+      for (int d = 0; d < 3; ++d) cs[d] = op.surf[3 * (row0 / 3 + gi) + d];
     }
-    __syncthreads();
-    if (!s_any) continue;
-    const bool par = op.mode == GEN_M2L && op.parent && t == op.nterms - 1;
-    const double *X = par ? op.X2 : op.X;
-    TermGeom g{};
-    if (op.mode != GEN_STORED) g = term_geom(op, oct, t);
-    for (int k0 = 0; k0 < op.K; k0 += GBK) {
-      if (op.mode == GEN_STORED) {
-        for (int e = tid; e < GBM * GBK; e += GTHREADS) {
-          const int r = e / GBK, kk = e % GBK;
-          const int row = row0 + r, k = k0 + kk;
-          As[kk][r] = (row < op.rows && k < op.K) ? op.A[static_cast<int64_t>(row) * op.lda + k] : 0.0;
+    int my_slot = -1;
+    if (tid < GBN && col0 + tid < col_end) my_slot = op.cols ? op.cols[col0 + tid] : col0 + tid;
+    // on to the next term with a source (every thread); false when there is none
+    auto next_term = [&]() {
+      while (++pt < t_hi) {
+        const int b = pbuf ^ 1;
+        int s = -1;
+        if (tid < GBN) {
+          if (my_slot >= 0) s = source_slot(op, oct, my_slot, pt);
+          s_src[b][tid] = s;
+          const unsigned live = __ballot_sync(0xffffffffu, s >= 0);
+          if (lane == 0) s_live[b][warp] = live;
         }
-      } else {
-        // 32 check points x 8 equivalent points: one 3 x 4 block of K4 each
-        // (a warp takes 32 consecutive check points of one equivalent point)
-        for (int pp = tid; pp < (GBM / 3) * (GBK / 4); pp += GTHREADS) {
-          const int ci = pp % (GBM / 3), ei = pp / (GBM / 3);
-          const int cp = row0 / 3 + ci, ep = k0 / 4 + ei;
-          double v[3][4];
-          if (cp < op.n && ep < op.n) {
-            const double r0 = op.crad * op.surf[3 * cp] - (g.off[0] + g.erad * op.surf[3 * ep]);
-            const double r1 = op.crad * op.surf[3 * cp + 1] - (g.off[1] + g.erad * op.surf[3 * ep + 1]);
-            const double r2 = op.crad * op.surf[3 * cp + 2] - (g.off[2] + g.erad * op.surf[3 * ep + 2]);
-            const double ri = rsqrt_refined(fma(r0, r0, fma(r1, r1, r2 * r2)));
-            const double ri3 = ri * ri * ri;
-            const double r[3] = {r0, r1, r2};
+        if (!__syncthreads_or(s >= 0)) continue;
+        pbuf = b;
+        pk = 0;
+        const double *x = (op.mode == GEN_M2L && op.parent && pt == op.nterms - 1) ? op.X2 : op.X;
+        pv = 0;
 #pragma unroll
-            for (int i = 0; i < 3; ++i) {
-#pragma unroll
-              for (int j = 0; j < 3; ++j) v[i][j] = fma(r[i] * r[j], ri3, i == j ? ri : 0.0);
-              v[i][3] = r[i] * ri3 * g.qscale;
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < 3; ++i)
-#pragma unroll
-              for (int j = 0; j < 4; ++j) v[i][j] = 0.0;
+        for (int i = 0; i < 4; ++i) {
+          const int sc = s_src[b][16 * i + 4 * warp + (lane & 3)];
+          px[i] = x + (lane >> 2);
+          if (sc >= 0) {
+            px[i] += static_cast<int64_t>(sc) * op.ldx;
+            pv |= 1u << i;
           }
+        }
+        if (op.mode != GEN_STORED)
+          pg = term_geom(op, oct, pt);
+        else
+          pa = op.A + static_cast<int64_t>(row0 + tid / GBK) * op.lda + tid % GBK;
+        return true;
+      }
+      return false;
+    };
+    // chunk (pt, pk) into buffer `buf`
+    auto produce = [&](int buf) {
+      const int k0 = GBK * pk;
+      // a warp gathers 4 boxes x 8 consecutive k (64-byte runs of each box's
+      // densities); its stores then fill the 16 bank pairs twice over
+      // (4 kk + c over the stride 4 mod 16), the minimum for 256 bytes.  K is a
+      // multiple of 8: the last chunk may end after any of its runs.
+      double *xs = &Xs[buf][lane >> 2][4 * warp + (lane & 3)];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const bool v = (pv >> i) & 1u;
+#pragma unroll
+        for (int q = 0; q < GBK / 8; ++q) {
+          const bool in = k0 + 8 * q < op.K;
+          cp_async8z(xs + 16 * i + 8 * q * GXS, in ? px[i] + 8 * q : px[i], v && in);
+        }
+        px[i] += GBK;
+      }
+      if (op.mode == GEN_STORED) {
+        const bool kv = k0 + tid % GBK < op.K;
+#pragma unroll
+        for (int i = 0; i < GBM * GBK / GTHREADS; ++i) {
+          const int r = tid / GBK + i * (GTHREADS / GBK);
+          const bool v = kv && row0 + r < op.rows;
+          cp_async8z(&As[buf][tid % GBK][r], v ? pa + static_cast<int64_t>(i * (GTHREADS / GBK)) * op.lda : op.A, v);
+        }
+        pa += GBK;
+      } else {
+        // one 3 x 4 block of K4
+        const int ep = k0 / 4 + ge;
+        double v[3][4];
+        if (gv && ep < op.n) {
+          double r[3];
+#pragma unroll
+          for (int d = 0; d < 3; ++d) r[d] = fma(op.crad, cs[d], -fma(pg.erad, op.surf[3 * ep + d], pg.off[d]));
+          const double ri = rsqrt_refined(fma(r[0], r[0], fma(r[1], r[1], r[2] * r[2])));
+          const double ri3 = ri * ri * ri;
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+#pragma unroll
+            for (int j = 0; j < 3; ++j) v[i][j] = fma(r[i] * r[j], ri3, i == j ? ri : 0.0);
+            v[i][3] = r[i] * ri3 * pg.qscale;
+          }
+        } else {
 #pragma unroll
           for (int i = 0; i < 3; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) As[4 * ei + j][3 * ci + i] = v[i][j];
+            for (int j = 0; j < 4; ++j) v[i][j] = 0.0;
         }
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) As[buf][4 * ge + j][3 * gi + i] = v[i][j];
       }
-      // a warp gathers 4 boxes x 8 consecutive k (64-byte runs of each box's
-      // densities); its stores then fill the 16 bank pairs twice over
-      // (4 kk + c over the stride 4 mod 16), the minimum for 256 bytes
-      for (int e = tid; e < GBN * GBK; e += GTHREADS) {
-        const int blk = e >> 5;
-        const int c = 4 * (blk % (GBN / 4)) + (e & 3);
-        const int kk = 8 * (blk / (GBN / 4)) + ((e >> 2) & 7);
-        const int s = s_src[c], k = k0 + kk;
-        Xs[kk][c] = (s >= 0 && k < op.K) ? X[static_cast<int64_t>(s) * op.ldx + k] : 0.0;
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+
+    bool more = next_term();
+    unsigned live = 0;
+    int cur_t = -1;
+    if (more) produce(0);
+    for (int buf = 0; more; buf ^= 1) {
+      // the chunk about to be multiplied
+      if (pt != cur_t) {
+        cur_t = pt;
+        live = s_live[pbuf][warp >> 1] >> (16 * (warp & 1));
       }
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
       __syncthreads();
+      // the next one (the other parity takes the next term's sources, so none
+      // is overwritten before its term's last chunk is produced)
+      if (++pk == chunks) more = next_term();
+      if (more) produce(buf ^ 1);
 #pragma unroll
       for (int ks = 0; ks < GBK; ks += 16) {
-        double bf[4][4];
+        double bf[2][4];
 #pragma unroll
-        for (int ni = 0; ni < 4; ++ni)
+        for (int ni = 0; ni < 2; ++ni)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) bf[ni][j] = Xs[ks + t4 + 4 * j][wc + 8 * ni + lg];
+          for (int j = 0; j < 4; ++j) bf[ni][j] = Xs[buf][ks + t4 + 4 * j][wc + 8 * ni + lg];
 #pragma unroll
         for (int mi = 0; mi < 3; ++mi) {
           double af[8];
 #pragma unroll
-          for (int q = 0; q < 8; ++q) af[q] = As[ks + t4 + 4 * (q >> 1)][wr + 16 * mi + lg + 8 * (q & 1)];
+          for (int q = 0; q < 8; ++q) af[q] = As[buf][ks + t4 + 4 * (q >> 1)][16 * mi + lg + 8 * (q & 1)];
 #pragma unroll
-          for (int ni = 0; ni < 4; ++ni) mma_f64_16816(acc[mi][ni], af, bf[ni]);
+          for (int ni = 0; ni < 2; ++ni)
+            if ((live >> (8 * ni)) & 255u) mma_f64_16816(acc[mi][ni], af, bf[ni]);
         }
       }
-      __syncthreads();
     }
+#pragma unroll
+    for (int ni = 0; ni < 2; ++ni)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int col = col0 + wc + 8 * ni + 2 * t4 + e;
+        if (col >= col_end) continue;
+        const int slot = op.cols ? op.cols[col] : col;
+        double *y = op.nsplit > 1 ? op.partial + (static_cast<int64_t>(split) * op.nslots + slot) * op.ldy
+                                  : op.Y + static_cast<int64_t>(slot) * op.ldy;
+#pragma unroll
+        for (int mi = 0; mi < 3; ++mi)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int row = row0 + 16 * mi + lg + 8 * h;
+            if (row >= op.rows) continue;
+            const double v = acc[mi][ni][2 * h + e];
+            if (op.nsplit > 1)
+              y[row] = v;
+            else
+              y[row] = op.accumulate ? fma(op.scale, v, y[row]) : op.scale * v;
+          }
+      }
+    __syncthreads();  // the next item's first chunk and sources overwrite this one's
   }
-#pragma unroll
-  for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int col = col0 + wc + 8 * ni + 2 * t4 + e;
-      if (col >= col_end) continue;
-      const int slot = op.cols ? op.cols[col] : col;
-      double *y = op.nsplit > 1 ? op.partial + (static_cast<int64_t>(blockIdx.z) * op.nslots + slot) * op.ldy
-                                : op.Y + static_cast<int64_t>(slot) * op.ldy;
-#pragma unroll
-      for (int mi = 0; mi < 3; ++mi)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int row = row0 + wr + 16 * mi + lg + 8 * h;
-          if (row >= op.rows) continue;
-          const double v = acc[mi][ni][2 * h + e];
-          if (op.nsplit > 1)
-            y[row] = v;
-          else
-            y[row] = op.accumulate ? fma(op.scale, v, y[row]) : op.scale * v;
-        }
-    }
 }
 
 // Y[slot][row] (+)= scale * sum over splits of the partials, in split order
@@ -1261,9 +1357,10 @@ int launch_gemm(GemmOp op, const int *group_start, DevBuf &partial, cudaStream_t
   }
   op.oct_col_start[8] = group_start ? group_start[8] : op.ncols;
   if (tiles > 65535) return F3D_ERR_TOO_LARGE;  // more boxes in a level than one launch covers
-  const int rtiles = (op.rows + GBM - 1) / GBM;
+  // (the split count is that of the 96-row tiles it was first chosen for)
+  const int stiles = (op.rows + kSplitRows - 1) / kSplitRows;
   const int64_t want = 4 * static_cast<int64_t>(sm_count());
-  int nsplit = static_cast<int>(std::min<int64_t>({(want + int64_t(rtiles) * tiles - 1) / (int64_t(rtiles) * tiles),
+  int nsplit = static_cast<int>(std::min<int64_t>({(want + int64_t(stiles) * tiles - 1) / (int64_t(stiles) * tiles),
                                                    int64_t(op.nterms), int64_t(32)}));
   const size_t per_split = static_cast<size_t>(op.nslots) * op.ldy * sizeof(double);
   nsplit = std::max(1, std::min<int>(nsplit, static_cast<int>((size_t(256) << 20) / std::max<size_t>(per_split, 1))));
@@ -1273,8 +1370,20 @@ int launch_gemm(GemmOp op, const int *group_start, DevBuf &partial, cudaStream_t
     if (rc) return rc;
     op.partial = as<double>(partial);
   }
-  const dim3 grid(static_cast<unsigned>(rtiles), static_cast<unsigned>(tiles), static_cast<unsigned>(nsplit));
-  fmm_gemm_kernel<<<grid, GTHREADS, 0, st>>>(op);
+  const int rtiles = (op.rows + GBM - 1) / GBM;
+  const int64_t items = static_cast<int64_t>(rtiles) * tiles * nsplit;
+  constexpr size_t smem = 2 * GBK * (GAS + GXS) * sizeof(double);
+  static bool attr[64] = {false};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return F3D_ERR_CUDA;
+  if (!attr[dev]) {
+    if (cudaFuncSetAttribute(fmm_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) !=
+        cudaSuccess)
+      return F3D_ERR_CUDA;
+    attr[dev] = true;
+  }
+  const unsigned grid = static_cast<unsigned>(std::min<int64_t>(items, 3 * static_cast<int64_t>(sm_count())));
+  fmm_gemm_kernel<<<grid, GTHREADS, smem, st>>>(op, rtiles, tiles);
   ++*launches;
   if (nsplit > 1) {
     const int64_t ne = static_cast<int64_t>(op.nslots) * op.rows;
