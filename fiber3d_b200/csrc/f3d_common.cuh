@@ -93,6 +93,16 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
   }
 }
 
+// 16 bytes global -> shared (cp.async); groups of such copies and their waits.
+__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(smem)), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 // D += A B on the FP64 tensor cores for one 16 x 8 x 16 step
 // (mma.sync.m16n8k16.f64): a[i] holds A(g + 8 (i & 1), t + 4 (i >> 1)),
 // b[j] holds B(t + 4 j, g), d[i] holds D(g + 8 (i >> 1), 2 t + (i & 1)), with
@@ -104,6 +114,14 @@ __device__ __forceinline__ void mma_f64_16816(double (&d)[4], const double (&a)[
       : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
       : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(a[4]), "d"(a[5]), "d"(a[6]), "d"(a[7]), "d"(b[0]),
         "d"(b[1]), "d"(b[2]), "d"(b[3]));
+}
+
+// The same for one 16 x 8 x 4 step: a0, a1 hold A(g, t) and A(g + 8, t), b holds B(t, g).
+__device__ __forceinline__ void mma_f64_1684(double (&d)[4], double a0, double a1, double b) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+      : "d"(a0), "d"(a1), "d"(b));
 }
 
 // 1/x for the pivot: the hardware approximation (rcp.approx.ftz.f64, about

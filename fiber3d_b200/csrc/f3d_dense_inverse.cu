@@ -62,15 +62,6 @@ constexpr int kGuABuf = kGjB * kGuAS, kGuBBuf = kGuKC * kGuBS;
 constexpr size_t kGjSmemUpdate =
     static_cast<size_t>(kGuStages) * (static_cast<size_t>(kGuABuf) + kGuBBuf) * sizeof(double);
 
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(smem)), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
 struct GjArgs {
   double *A;        // np x np (leading dimension ld), np a multiple of 128
   const double *R;  // 128 x ld: the step's block row before the step

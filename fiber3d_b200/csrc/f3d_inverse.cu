@@ -30,6 +30,7 @@
 // (batched_inverse_tc_kernel): 16-column panels, no row exchanges, and the
 // rank-16 updates on the FP64 tensor cores.
 #include <algorithm>
+#include <climits>
 
 #include "f3d_common.cuh"
 
@@ -228,23 +229,34 @@ __global__ void __launch_bounds__(InvShape<NMAX>::kThreads, 1)
   }
 }
 
-// Blocked Gauss-Jordan for blocks of 33..128 rows (NMAX 64 or 128): one CTA
+// Blocked Gauss-Jordan for blocks of 33..128 rows (NMAX 64, 96 or 128): one CTA
 // per block, the block in shared memory (padded with the identity), 16
 // pivots per panel.
-//  * Panel: NMAX threads, one row each with the row's 16 panel entries in
-//    registers, run the 16 sweeps restricted to the panel columns.  Partial
-//    pivoting: the pivot of step k is the first row whose |a_ik|, rounded
-//    toward zero to float with its last 8 mantissa bits cleared, is largest
-//    among the rows not yet pivoted (a pivot within 2^-16 of the column
+//  * Panel: four sub-panels of 4 columns.  NMAX threads, one row each with
+//    the row's 4 entries in registers, run the 4 sweeps; the panel's other 12
+//    columns then move by W R of the sub-panel, one m16n8k4 step per 16 x 8
+//    tile.  (The chain of pivots bounds the kernel, and with all 16 columns
+//    in registers a step is bound by the shared-memory pipe: each warp's best
+//    row is posted and the pivot row read back 16 bytes at a time, about five
+//    cycles an access and warp.)  Partial pivoting: the pivot of step k is the
+//    first row whose |a_ik|, cut to its leading 12 mantissa bits, is largest
+//    among the rows not yet pivoted (a pivot within 2^-12 of the column
 //    maximum).  The key (those bits, then 128 - row) makes the search one
 //    warp max-reduction and a max over the warps; each warp's winner posts
-//    its row with its key, so a step needs one barrier (posts double
+//    its row, key and reciprocal, so a step needs one barrier (posts double
 //    buffered by step parity).  Rows are never exchanged: the pivot rows are
 //    recorded instead (perm).
 //  * Update: every other column moves by W R (W the panel after its sweeps,
 //    R the old entries of the panel's 16 pivot rows), the pivot rows
 //    themselves starting from zero: one m16n8k16 step on the FP64 tensor
-//    cores per 16 x 8 tile.
+//    cores per 16 x 8 tile.  At 128 rows (172 KB: one block per SM) the next
+//    panel's columns come first, by all warps, then the rest by half of them
+//    while the others sweep that panel; up to 96 rows two blocks share an SM
+//    and up to 64 rows four, which overlap by themselves.
+// 512 blocks: 250 us at 128 rows, 115 at 96, 45 at 64, against 307, 286 (by the
+// 128-row kernel) and 71 us with 16-column sweeps in registers and the update
+// after them; one block of 128: 65 us, 78 before.  (The block in global memory
+// with four CTAs per SM: 266 us.)
 // Sweeping pivot (perm[k], k) for every k leaves X with X[perm[k], j] =
 // (PA)^-1 (k, j), so A^-1 (k, perm[j]) = X[perm[k], j].
 template <int NMAX>
@@ -253,13 +265,15 @@ struct TcInv {
   static constexpr int kWS = 20;       // W panel row stride: A-fragment reads 4g + t apart
   static constexpr int kPanels = NMAX / 16;
   static constexpr int kThreads = 256;
+  static constexpr bool kAhead = NMAX > 96;      // sweep the next panel beside the update: one block per SM
+  static constexpr int kW = kAhead ? 2 : 1;      // W panels held
   static constexpr size_t kSmem =
-      (static_cast<size_t>(NMAX) * kS + static_cast<size_t>(NMAX) * kWS + 16 * static_cast<size_t>(kS)) *
+      (static_cast<size_t>(NMAX) * kS + kW * static_cast<size_t>(NMAX) * kWS + 16 * static_cast<size_t>(kS)) *
       sizeof(double);
 };
 
 template <int NMAX>
-__global__ void __launch_bounds__(256, 1)
+__global__ void __launch_bounds__(256, NMAX == 64 ? 4 : (NMAX == 96 ? 2 : 1))
     batched_inverse_tc_kernel(double *__restrict__ A, const int64_t *__restrict__ moff,
                               const int32_t *__restrict__ sizes, int count, float *__restrict__ A32,
                               int32_t *__restrict__ info) {
@@ -267,129 +281,207 @@ __global__ void __launch_bounds__(256, 1)
   constexpr int S = T::kS;
   extern __shared__ __align__(16) unsigned char tc_smem[];
   double *X = reinterpret_cast<double *>(tc_smem);  // [NMAX][S]
-  double *Ws = X + NMAX * S;                         // [NMAX][kWS]
-  double *Rs = Ws + NMAX * T::kWS;                   // [16][S]
-  __shared__ unsigned s_key[2][NMAX / 32];
-  __shared__ __align__(16) double s_cand[2][NMAX / 32][16];  // each warp's best row, by step parity
+  double *W2 = X + NMAX * S;                         // [kW][NMAX][kWS], by panel parity
+  double *Rs = W2 + T::kW * NMAX * T::kWS;           // [16][S]
+  __shared__ __align__(16) unsigned s_key[2][4];
+  __shared__ __align__(16) double s_cand[2][NMAX / 32][6];  // each warp's best row of the sub-panel and its
+                                                            // pivot's reciprocal, by step parity
+  __shared__ int s_zero;
   __shared__ int s_perm[NMAX];   // pivot row of step k
-  __shared__ int s_iperm[NMAX];  // step whose pivot is row r
-  __shared__ int s_panel[NMAX];  // panel in which row r was a pivot (-1: not yet)
+  __shared__ int s_step[NMAX];   // step whose pivot is row r (-16: not yet)
   const int b = blockIdx.x;
   if (b >= count) return;
   const int n = sizes[b];
   if (n <= 0 || n > NMAX) return;
   double *M = A + moff[b];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int e = tid; e < NMAX * NMAX; e += T::kThreads) {
-    const int r = e / NMAX, c = e % NMAX;
-    X[r * S + c] = (r < n && c < n) ? M[static_cast<int64_t>(r) * n + c] : (r == c ? 1.0 : 0.0);
+  if (n == NMAX && (reinterpret_cast<uintptr_t>(M) & 15) == 0) {
+    for (int e = tid; e < NMAX * NMAX / 2; e += T::kThreads)
+      cp_async16(&X[e / (NMAX / 2) * S + 2 * (e % (NMAX / 2))], M + 2 * e);
+    cp_async_commit();
+    cp_async_wait<0>();
+  } else {
+#pragma unroll 4
+    for (int e = tid; e < NMAX * NMAX; e += T::kThreads) {
+      const int r = e / NMAX, c = e % NMAX;
+      X[r * S + c] = (r < n && c < n) ? M[static_cast<int64_t>(r) * n + c] : (r == c ? 1.0 : 0.0);
+    }
   }
-  for (int r = tid; r < NMAX; r += T::kThreads) s_panel[r] = -1;
+  for (int r = tid; r < NMAX; r += T::kThreads) s_step[r] = -16;
+  if (tid < 8) s_key[tid >> 2][tid & 3] = 0u;
+  if (tid == 0) s_zero = INT_MAX;
   __syncthreads();
-  int first_zero = 0;  // kept by thread 0
-  for (int p = 0; p < T::kPanels; ++p) {
-    const int c0 = 16 * p;
-    if (tid < NMAX) {
-      const int i = tid;
-      double v[16];
+  int first_zero = 0;  // the first zero pivot this thread's row was (a row is a pivot once)
+  bool done = false;   // this thread's row has been a pivot
+  constexpr int kRT = NMAX / 16, kCT = NMAX / 8, kPW = NMAX / 32;
+  const int g = lane >> 2, t = lane & 3;
+
+  // panel p (warps 0 .. kPW - 1): its sweeps, W to its buffer and to the panel's columns
+  auto panel = [&](int p) {
+    const int c0 = 16 * p, i = tid;
+    double *Ws = W2 + (T::kAhead ? p & 1 : 0) * NMAX * T::kWS;
+    auto bar = [] { asm volatile("bar.sync 1, %0;" ::"n"(NMAX) : "memory"); };
 #pragma unroll
-      for (int j = 0; j < 16; ++j) v[j] = X[i * S + c0 + j];
-      bool done = s_panel[i] >= 0;
+    for (int j = 0; j < 16; j += 2)
+      *reinterpret_cast<double2 *>(&Ws[i * T::kWS + j]) = *reinterpret_cast<const double2 *>(&X[i * S + c0 + j]);
+    for (int s0 = 0; s0 < 16; s0 += 4) {
+      double v[4];
 #pragma unroll
-      for (int jj = 0; jj < 16; ++jj) {
-        const int par = jj & 1;
-        // pivot key: |a_ik| as a float rounded toward zero, last 8 mantissa
-        // bits replaced by 128 - row (first row among equals; never 0 for a
-        // row not yet pivoted); pivoted rows 0
-        const unsigned key =
-            done ? 0u : ((__float_as_uint(__double2float_rz(fabs(v[jj]))) & ~255u) | static_cast<unsigned>(128 - i));
+      for (int j = 0; j < 4; j += 2) {
+        const double2 w = *reinterpret_cast<const double2 *>(&Ws[i * T::kWS + s0 + j]);
+        v[j] = w.x;
+        v[j + 1] = w.y;
+      }
+      int piv[4];  // the sub-panel's pivot rows
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+        const int par = jj & 1, k = c0 + s0 + jj;
+        // pivot key: the leading word of |a_ik|, its last 8 bits replaced by
+        // 128 - row (first row among equals; never 0 for a row not yet
+        // pivoted); pivoted rows 0
+        const unsigned key = done ? 0u
+                                  : ((static_cast<unsigned>(__double2hiint(v[jj])) & 0x7fffff00u) |
+                                     static_cast<unsigned>(128 - i));
+        const double rcp = reciprocal(v[jj]);  // beside the search
         const unsigned wmax = __reduce_max_sync(0xffffffffu, key);
         if (key == wmax) {  // this warp's winner posts its row (live keys are distinct; a warp
                             // with no live row posts garbage under key 0, which never wins)
           s_key[par][warp] = wmax;
-#pragma unroll
-          for (int j = 0; j < 16; ++j) s_cand[par][warp][j] = v[j];
+          double *const c = s_cand[par][warp];
+          *reinterpret_cast<double2 *>(c) = make_double2(v[0], v[1]);
+          *reinterpret_cast<double2 *>(c + 2) = make_double2(v[2], v[3]);
+          c[4] = rcp;
         }
-        asm volatile("bar.sync 1, %0;" ::"r"(NMAX) : "memory");
-        unsigned best = s_key[par][0];
-        int bw = 0;
-#pragma unroll
-        for (int w = 1; w < NMAX / 32; ++w)
-          if (s_key[par][w] > best) {
-            best = s_key[par][w];
-            bw = w;
-          }
+        bar();
+        const uint4 h = *reinterpret_cast<const uint4 *>(s_key[par]);
+        const unsigned best = max(max(h.x, h.y), max(h.z, h.w));
         const int pr = 128 - static_cast<int>(best & 255u);
-        const double *prow = s_cand[par][bw];
+        piv[jj] = pr;
+        const double *prow = s_cand[par][pr >> 5];
+        const double inv = prow[4];
         if (i == pr) {
-          s_perm[c0 + jj] = i;
-          s_panel[i] = p;
+          s_perm[k] = i;
+          s_step[i] = k;
           done = true;
-        }
-        const double d = prow[jj];
-        if (tid == 0 && first_zero == 0 && !(fabs(d) >= 2.2250738585072014e-308)) first_zero = c0 + jj + 1;
-        const double inv = reciprocal(d);
-        if (i == pr) {
+          if (first_zero == 0 && !(fabs(v[jj]) >= 2.2250738585072014e-308)) first_zero = k + 1;
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = (j == jj) ? inv : v[j] * inv;
+          for (int j = 0; j < 4; ++j) v[j] = (j == jj) ? inv : v[j] * inv;
         } else {
           const double l = v[jj] * inv;
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = (j == jj) ? -l : fma(-l, prow[j], v[j]);
+          for (int j = 0; j < 4; ++j) v[j] = (j == jj) ? -l : fma(-l, prow[j], v[j]);
         }
       }
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        X[i * S + c0 + j] = v[j];
-        Ws[i * T::kWS + j] = v[j];
+      for (int j = 0; j < 4; j += 2)
+        *reinterpret_cast<double2 *>(&Ws[i * T::kWS + s0 + j]) = make_double2(v[j], v[j + 1]);
+      bar();
+      // the panel's other 12 columns: one m16n8k4 step per 16 x 8 tile (four
+      // tiles a warp, row tiles first), the four pivot rows taken into registers
+      // before any of them changes
+      const int pt = t == 0 ? piv[0] : (t == 1 ? piv[1] : (t == 2 ? piv[2] : piv[3]));
+      double2 o[4][2];
+      double af[4][2], b4[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int id = 4 * warp + q, rt = id % kRT, ch = 8 * (id / kRT);
+        b4[q] = Ws[pt * T::kWS + ch + g];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int r = 16 * rt + g + 8 * h;
+          const bool keep = r != piv[0] && r != piv[1] && r != piv[2] && r != piv[3];
+          const double2 x = *reinterpret_cast<const double2 *>(&Ws[r * T::kWS + ch + 2 * t]);
+          o[q][h] = keep ? x : make_double2(0.0, 0.0);
+          af[q][h] = Ws[r * T::kWS + s0 + t];
+        }
+      }
+      bar();
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int id = 4 * warp + q, rt = id % kRT, cc = 8 * (id / kRT) + 2 * t;
+        double dd[4] = {o[q][0].x, o[q][0].y, o[q][1].x, o[q][1].y};
+        mma_f64_1684(dd, af[q][0], af[q][1], b4[q]);
+        if ((cc & ~3) != s0) {  // (the sub-panel's own columns hold its W)
+          double *x = &Ws[(16 * rt + g) * T::kWS + cc];
+          *reinterpret_cast<double2 *>(x) = make_double2(dd[0], dd[1]);
+          *reinterpret_cast<double2 *>(x + 8 * T::kWS) = make_double2(dd[2], dd[3]);
+        }
+      }
+      bar();
+    }
+#pragma unroll
+    for (int j = 0; j < 16; j += 2)
+      *reinterpret_cast<double2 *>(&X[i * S + c0 + j]) = *reinterpret_cast<const double2 *>(&Ws[i * T::kWS + j]);
+  };
+  // panel p's update of row tile rt, column tiles ct = ct0, ct0 + step, ...
+  // outside the panels p and `skip`: X <- [row not a pivot of this panel] X + W R
+  auto update = [&](int p, int skip, int rt, int ct0, int ct1, int step) {
+    const double *Ws = W2 + (T::kAhead ? p & 1 : 0) * NMAX * T::kWS;
+    const int r0 = 16 * rt + g, r1 = r0 + 8;
+    double af[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) af[q] = Ws[(r0 + 8 * (q & 1)) * T::kWS + t + 4 * (q >> 1)];
+    const bool keep0 = (s_step[r0] >> 4) != p, keep1 = (s_step[r1] >> 4) != p;
+    for (int ct = ct0; ct < ct1; ct += step) {
+      if ((ct >> 1) == p || (ct >> 1) == skip) continue;
+      const int c = 8 * ct;
+      double bf[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) bf[j] = Rs[(t + 4 * j) * S + c + g];
+      double2 *x0 = reinterpret_cast<double2 *>(X + r0 * S + c + 2 * t);
+      double2 *x1 = reinterpret_cast<double2 *>(X + r1 * S + c + 2 * t);
+      const double2 o0 = *x0, o1 = *x1;
+      double dd[4] = {keep0 ? o0.x : 0.0, keep0 ? o0.y : 0.0, keep1 ? o1.x : 0.0, keep1 ? o1.y : 0.0};
+      mma_f64_16816(dd, af, bf);
+      *x0 = make_double2(dd[0], dd[1]);
+      *x1 = make_double2(dd[2], dd[3]);
+    }
+  };
+
+  auto all_but = [&](int p, int skip, int w0) {  // warps w0 .. 7: column tiles of one parity each
+    for (int it = warp - w0; it < 2 * kRT; it += 8 - w0) update(p, skip, it >> 1, it & 1, kCT, 2);
+  };
+
+  if (warp < kPW) panel(0);
+  for (int p = 0; p < T::kPanels; ++p) {
+    __syncthreads();
+    // the panel's pivot rows as they were before the panel (outside its columns)
+    for (int e = tid; e < 16 * NMAX / 2; e += T::kThreads) {
+      const int jj = e / (NMAX / 2), c = 2 * (e % (NMAX / 2));
+      if ((c >> 4) != p)
+        *reinterpret_cast<double2 *>(&Rs[jj * S + c]) =
+            *reinterpret_cast<const double2 *>(&X[s_perm[16 * p + jj] * S + c]);
+    }
+    __syncthreads();
+    if (T::kAhead && p + 1 < T::kPanels) {
+      // the next panel's columns first, so that its sweeps run beside the rest
+      if (warp < kRT) update(p, -1, warp, 2 * (p + 1), 2 * (p + 2), 1);
+      __syncthreads();
+      if (warp < kPW)
+        panel(p + 1);
+      else
+        all_but(p, p + 1, kPW);
+    } else {
+      all_but(p, -1, 0);
+      if (p + 1 < T::kPanels) {
+        __syncthreads();
+        if (warp < kPW) panel(p + 1);
       }
     }
-    __syncthreads();
-    // the panel's pivot rows as they were before the panel
-    for (int e = tid; e < 16 * NMAX; e += T::kThreads) {
-      const int jj = e / NMAX, c = e % NMAX;
-      Rs[jj * S + c] = X[s_perm[c0 + jj] * S + c];
-    }
-    __syncthreads();
-    // every column tile outside the panel: X <- [row not a pivot of this
-    // panel] X + W R, on the tensor cores
-    {
-      constexpr int kRT = NMAX / 16, kCT = NMAX / 8, kStride = 8 / kRT;
-      const int g = lane >> 2, t = lane & 3;
-      const int rt = warp % kRT;
-      const int r0 = 16 * rt + g, r1 = r0 + 8;
-      double af[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) af[q] = Ws[(16 * rt + g + 8 * (q & 1)) * T::kWS + t + 4 * (q >> 1)];
-      const bool keep0 = s_panel[r0] != p, keep1 = s_panel[r1] != p;
-      for (int ct = warp / kRT; ct < kCT; ct += kStride) {
-        if ((ct >> 1) == p) continue;  // the panel's own two column tiles
-        const int c = 8 * ct;
-        double bf[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) bf[j] = Rs[(t + 4 * j) * S + c + g];
-        double2 *x0 = reinterpret_cast<double2 *>(X + r0 * S + c + 2 * t);
-        double2 *x1 = reinterpret_cast<double2 *>(X + r1 * S + c + 2 * t);
-        const double2 o0 = *x0, o1 = *x1;
-        double dd[4] = {keep0 ? o0.x : 0.0, keep0 ? o0.y : 0.0, keep1 ? o1.x : 0.0, keep1 ? o1.y : 0.0};
-        mma_f64_16816(dd, af, bf);
-        *x0 = make_double2(dd[0], dd[1]);
-        *x1 = make_double2(dd[2], dd[3]);
-      }
-    }
-    __syncthreads();
   }
-  // A^-1 (k, c) = X[perm[k], iperm[c]]: coalesced stores of the block's rows
-  for (int k = tid; k < NMAX; k += T::kThreads) s_iperm[s_perm[k]] = k;
   __syncthreads();
+  // A^-1 (k, c) = X[perm[k], step[c]]: coalesced stores of the block's rows
   float *M32 = A32 ? A32 + moff[b] : nullptr;
   for (int e = tid; e < n * n; e += T::kThreads) {
     const int k = e / n, c = e % n;
-    const double v = X[s_perm[k] * S + s_iperm[c]];
+    const double v = X[s_perm[k] * S + s_step[c]];
     M[e] = v;
     if (M32) M32[e] = static_cast<float>(v);
   }
-  if (tid == 0) info[b] = first_zero;
+  // the first step whose pivot was zero, over the threads that held pivots
+  if (first_zero) atomicMin(&s_zero, first_zero);
+  __syncthreads();
+  if (tid == 0) info[b] = s_zero == INT_MAX ? 0 : s_zero;
 }
 
 // y_b = M_b x_b for every block b (M row-major n_b x n_b at moff[b], x and y
@@ -461,6 +553,13 @@ int f3d_batched_inverse(double *A, const int64_t *matrix_offsets, const int32_t 
                              static_cast<int>(T::kSmem)) != cudaSuccess)
       return F3D_ERR_CUDA;
     f3d::batched_inverse_tc_kernel<64><<<count, T::kThreads, T::kSmem, st>>>(A, matrix_offsets, sizes, count, A32,
+                                                                             info);
+  } else if (max_n <= 96) {
+    using T = f3d::TcInv<96>;
+    if (cudaFuncSetAttribute(f3d::batched_inverse_tc_kernel<96>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(T::kSmem)) != cudaSuccess)
+      return F3D_ERR_CUDA;
+    f3d::batched_inverse_tc_kernel<96><<<count, T::kThreads, T::kSmem, st>>>(A, matrix_offsets, sizes, count, A32,
                                                                              info);
   } else {
     using T = f3d::TcInv<128>;
