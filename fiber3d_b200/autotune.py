@@ -194,6 +194,20 @@ def cached(kernel: str, precision: str, self_mode: str, ns: int, nt: int,
     return _lib.PairShape(*v) if v is not None else None
 
 
+def key(kernel: str, precision: str, self_mode: str, ns: int, nt: int, same: bool = False) -> str:
+    """The cache key of a sum (its size buckets, on the current GPU)."""
+    return _key(kernel, precision, self_mode, ns, nt, same)
+
+
+def entry(cache_key: str) -> list | None:
+    """The cache's own entry under `cache_key`: a new object whenever that sum
+    is tuned again (a caller that kept one can tell by identity)."""
+    if not _loaded:
+        with _lock:
+            _load()
+    return _cache.get(cache_key)
+
+
 def table() -> dict:
     """The cached shapes (for reports)."""
     with _lock:
