@@ -147,6 +147,10 @@ int *device_error_word();
 // The limit (ns) that entry points hand to their kernels' bounded waits.
 uint64_t wait_limit_ns();
 
+// Inverse of one 128 x 128 block (f3d_inverse.cu).
+int pivot_block_inverse(const double *src, int64_t ld, double *Q, const int64_t *off, const int32_t *size,
+                        int32_t *info, cudaStream_t st);
+
 inline bool aligned(const void *p, uintptr_t a) {
   return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0;
 }

@@ -24,15 +24,14 @@
 // entries grow by at most 1.06 during elimination.  A zero pivot inside a
 // block is reported (F3D_ERR_SINGULAR).
 //
-// Per step: the pivot block is copied out and inverted (one CTA), the old
-// block row is copied to R, gj_panel_kernel forms W in place in the panel
-// columns (one CTA per 128-row tile, 8 x 8 FP64 FMA accumulators per
-// thread), and gj_update_kernel updates every other 128 x 128 tile on the
-// FP64 tensor cores: one persistent CTA per SM (8 warps of 64 x 32 outputs,
-// mma.sync m16n8k16) walks its tiles with one continuous stream of operand
-// chunks (32 k, cp.async, a three-stage ring, one barrier per chunk) across
-// tile boundaries; a tile's old values are prefetched into L2 when its first
-// chunk is requested and added in its epilogue.
+// Per step: the pivot block is inverted (one CTA); gj_panel_kernel forms W in
+// place in the panel columns and copies the old block row to R (a CTA per 32
+// rows); gj_update_kernel updates every other tile; both on the FP64 tensor
+// cores (mma.sync m16n8k16).  The update is persistent, two CTAs per SM (4
+// warps of 32 x 64 outputs, tiles of 64 x 128), each walking its tiles with one
+// continuous stream of operand chunks (32 k, cp.async, a two-stage ring, one
+// barrier per chunk) across tile boundaries; a tile's old values are prefetched
+// into L2 when its first chunk is requested and added in its epilogue.
 #include <algorithm>
 #include <vector>
 
@@ -42,137 +41,145 @@ namespace f3d {
 namespace {
 
 constexpr int kGjB = 128;             // rows/columns of a step and of a tile
-constexpr int kGjKC = 16;             // k per staged chunk
-constexpr int kGjChunks = kGjB / kGjKC;
-constexpr int kGjThreads = 256;       // 16 x 16 threads, 8 x 8 outputs each
-constexpr int kGjAStride = kGjKC + 2; // padded row of the m-major operand chunk (144 B)
-constexpr int kGjABuf = kGjB * kGjAStride;
-constexpr int kGjBBuf = kGjKC * kGjB;
-constexpr size_t kGjSmemPanel = (2 * kGjABuf + 2 * kGjBBuf) * sizeof(double);
-// update: 256 threads, 8 warps of 64 x 32 outputs on the FP64 tensor cores
-// (mma.sync m16n8k16), operands in a three-stage ring of 32-k chunks.
+// panel: 128 threads, 4 warps of 16 x 64 outputs, 32 rows per CTA; operand
+// strides as the update's below
+constexpr int kGpThreads = 128;
+constexpr int kGpM = 32;
+// update: 128 threads, 4 warps of 32 x 64 outputs on the FP64 tensor cores
+// (mma.sync m16n8k16), operands in a two-stage ring of 32-k chunks.
 // Shared row strides (doubles) chosen so that every fragment read is two
-// conflict-free wavefronts: W chunk [128][36] (row-major A fragments: 4g + t
+// conflict-free wavefronts: W chunk [64][36] (row-major A fragments: 4g + t
 // distinct mod 16 over a half-warp), R chunk [32][132] (k-major B
 // fragments: 4t + g).
-constexpr int kGuThreads = 256;
-constexpr int kGuKC = 32, kGuChunks = kGjB / kGuKC, kGuStages = 3;
+constexpr int kGuThreads = 128;
+constexpr int kGuM = 64;  // rows of an update tile (128 columns)
+constexpr int kGuKC = 32, kGuChunks = kGjB / kGuKC, kGuStages = 2;
 constexpr int kGuAS = 36, kGuBS = 132;
-constexpr int kGuABuf = kGjB * kGuAS, kGuBBuf = kGuKC * kGuBS;
+constexpr int kGuABuf = kGuM * kGuAS, kGuBBuf = kGuKC * kGuBS;
 constexpr size_t kGjSmemUpdate =
     static_cast<size_t>(kGuStages) * (static_cast<size_t>(kGuABuf) + kGuBBuf) * sizeof(double);
+constexpr int kGpABuf = kGpM * kGuAS;
+constexpr size_t kGjSmemPanel = 2 * (static_cast<size_t>(kGpABuf) + kGuBBuf) * sizeof(double);
 
 struct GjArgs {
   double *A;        // np x np (leading dimension ld), np a multiple of 128
-  const double *R;  // 128 x ld: the step's block row before the step
+  double *R;        // 128 x ld: the step's block row before the step
   const double *Q;  // 128 x 128: inverse of the step's pivot block
   int64_t ld;
   int s;            // step: pivot block index
   int *err;         // the device error word (read by the host after the last step)
 };
 
-// Thread (tx, ty) owns rows 2ty + 32q + e and columns 2tx + 32q + e
-// (q < 4, e < 2) of its tile: pairs of adjacent columns for 16-byte accesses,
-// the pairs of a warp contiguous (conflict-free shared-memory reads).
-
-// Chunk c of a tile's operands into buffer `buf`: A(row0 + m, k0 + 16c + kk)
-// (the step's panel columns) and B(16c + kk, n) = bsrc[(16c + kk) * bld + n].
-__device__ __forceinline__ void gj_load_chunk(double *As, double *Bs, const double *A, int64_t ld, int64_t row0,
-                                              int64_t k0, const double *bsrc, int64_t bld, int c, int buf, int tid) {
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int seg = tid + u * kGjThreads;  // 128 rows x 8 segments of 16 B
-    const int m = seg >> 3, q = seg & 7;
-    cp_async16(As + buf * kGjABuf + m * kGjAStride + 2 * q, A + (row0 + m) * ld + k0 + c * kGjKC + 2 * q);
-  }
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int seg = tid + u * kGjThreads;  // 16 rows x 64 segments of 16 B
-    const int kk = seg >> 6, q = seg & 63;
-    cp_async16(Bs + buf * kGjBBuf + kk * kGjB + 2 * q, bsrc + static_cast<int64_t>(c * kGjKC + kk) * bld + 2 * q);
-  }
-  cp_async_commit();
-}
-
-// acc += A-chunk x B-chunk (16 k) from shared memory.
-__device__ __forceinline__ void gj_mma_chunk(double (&acc)[8][8], const double *as, const double *bs, int tx,
-                                             int ty) {
-#pragma unroll
-  for (int kk = 0; kk < kGjKC; ++kk) {
-    double av[8], bv[8];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int r = 2 * ty + 32 * q;
-      av[2 * q] = as[r * kGjAStride + kk];
-      av[2 * q + 1] = as[(r + 1) * kGjAStride + kk];
-      const double2 b2 = *reinterpret_cast<const double2 *>(bs + kk * kGjB + 2 * tx + 32 * q);
-      bv[2 * q] = b2.x;
-      bv[2 * q + 1] = b2.y;
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) acc[i][j] = fma(av[i], bv[j], acc[i][j]);
-  }
-}
-
-// The panel: W_I = -A(I, b) Q for row tiles I != s, W_s = Q, written in
-// place into the panel columns (one CTA per row tile).
-__global__ void __launch_bounds__(kGjThreads, 1) gj_panel_kernel(const GjArgs a) {
+// The panel: W_I = -A(I, b) Q for rows I outside the pivot block, W_s = Q,
+// written in place into the panel columns, on the FP64 tensor cores, 32 rows
+// per CTA; and the block row R as it was before the step, a 32 x 128 piece per
+// CTA.  32 rows leave enough CTAs for every SM from 37 tiles on, and a quarter
+// of the time of 128-row CTAs below that: 28 us a step at 10 and at 71 tiles
+// for 128 rows with FP64 FMAs, 9 and 16 us now, the copy of R (3.4 and 6.6 us)
+// included.
+__global__ void __launch_bounds__(kGpThreads, 2) gj_panel_kernel(const GjArgs a) {
   extern __shared__ __align__(16) unsigned char gj_smem[];
-  double *As = reinterpret_cast<double *>(gj_smem);  // [2][128][kGjAStride]: A[row][k]
-  double *Bs = As + 2 * kGjABuf;                      // [2][16][128]: Q[k][col]
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int I = blockIdx.x;
-  const int64_t row0 = static_cast<int64_t>(I) * kGjB, k0 = static_cast<int64_t>(a.s) * kGjB;
-  if (I == a.s) {
-    for (int i = tid; i < kGjB * kGjB / 2; i += kGjThreads) {
+  double *As = reinterpret_cast<double *>(gj_smem);  // [2][32][kGuAS]: A[row][k]
+  double *Bs = As + 2 * kGpABuf;                      // [2][32][kGuBS]: Q[k][col]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const int64_t row0 = static_cast<int64_t>(blockIdx.x) * kGpM, k0 = static_cast<int64_t>(a.s) * kGjB;
+  // this CTA's piece of R: rows 32 (x % 4) .. + 31 of the block, column tile x / 4
+  // (the panel's own columns are not read from R)
+  const int J = blockIdx.x / (kGjB / kGpM), rp = kGpM * (blockIdx.x % (kGjB / kGpM));
+  if (J != a.s) {
+    const double *src = a.A + (k0 + rp + (tid >> 6)) * a.ld + static_cast<int64_t>(J) * kGjB + 2 * (tid & 63);
+    double *dst = a.R + (rp + (tid >> 6)) * a.ld + static_cast<int64_t>(J) * kGjB + 2 * (tid & 63);
+    double2 v[kGpM / 2];
+#pragma unroll
+    for (int i = 0; i < kGpM / 2; ++i) v[i] = *reinterpret_cast<const double2 *>(src + 2 * i * a.ld);
+#pragma unroll
+    for (int i = 0; i < kGpM / 2; ++i) *reinterpret_cast<double2 *>(dst + 2 * i * a.ld) = v[i];
+  }
+  if (row0 >= k0 && row0 < k0 + kGjB) {
+    for (int i = tid; i < kGpM * kGjB / 2; i += kGpThreads) {
       const int r = i / (kGjB / 2), c2 = i % (kGjB / 2);
       reinterpret_cast<double2 *>(a.A + (row0 + r) * a.ld + k0)[c2] =
-          reinterpret_cast<const double2 *>(a.Q + r * kGjB)[c2];
+          reinterpret_cast<const double2 *>(a.Q + (row0 - k0 + r) * kGjB)[c2];
     }
     return;
   }
-  double acc[8][8];
+  auto load = [&](int c) {
+    double *as = As + (c & 1) * kGpABuf, *bs = Bs + (c & 1) * kGuBBuf;
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+    for (int v = 0; v < kGpM / 8; ++v) {  // 32 rows x 16 segments of 16 B
+      const int m = (tid >> 4) + 8 * v;
+      cp_async16(as + m * kGuAS + 2 * (tid & 15), a.A + (row0 + m) * a.ld + k0 + c * kGuKC + 2 * (tid & 15));
+    }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.0;
-  gj_load_chunk(As, Bs, a.A, a.ld, row0, k0, a.Q, kGjB, 0, 0, tid);
-  for (int c = 0; c < kGjChunks; ++c) {
+    for (int v = 0; v < kGuKC / 2; ++v) {  // 32 rows x 64 segments of 16 B
+      const int kk = (tid >> 6) + 2 * v;
+      cp_async16(bs + kk * kGuBS + 2 * (tid & 63), a.Q + (c * kGuKC + kk) * kGjB + 2 * (tid & 63));
+    }
+    cp_async_commit();
+  };
+  const int wr = 16 * (warp >> 1), wc = 64 * (warp & 1);
+  double acc[8][4];
+#pragma unroll
+  for (int ni = 0; ni < 8; ++ni)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[ni][i] = 0.0;
+  load(0);
+  for (int c = 0; c < kGuChunks; ++c) {
     cp_async_wait<0>();
     __syncthreads();
-    if (c + 1 < kGjChunks) gj_load_chunk(As, Bs, a.A, a.ld, row0, k0, a.Q, kGjB, c + 1, (c + 1) & 1, tid);
-    gj_mma_chunk(acc, As + (c & 1) * kGjABuf, Bs + (c & 1) * kGjBBuf, tx, ty);
+    if (c + 1 < kGuChunks) load(c + 1);
+#pragma unroll
+    for (int ks = 0; ks < kGuKC / 16; ++ks) {
+      const double *as = As + (c & 1) * kGpABuf + (wr + g) * kGuAS + 16 * ks + t;
+      const double *bs = Bs + (c & 1) * kGuBBuf + (16 * ks + t) * kGuBS + wc + g;
+      double af[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) af[i] = as[8 * (i & 1) * kGuAS + 4 * (i >> 1)];
+#pragma unroll
+      for (int ni = 0; ni < 8; ++ni) {
+        double bf[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) bf[j] = bs[4 * j * kGuBS + 8 * ni];
+        mma_f64_16816(acc[ni], af, bf);
+      }
+    }
   }
+  // (every thread's last reads of A were the copies waited for before the last barrier)
+  double *o = a.A + (row0 + wr + g) * a.ld + k0 + wc + 2 * t;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int r = 2 * ty + 32 * (i >> 1) + (i & 1);
-    double *o = a.A + (row0 + r) * a.ld + k0;
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-      *reinterpret_cast<double2 *>(o + 2 * tx + 32 * q) = make_double2(-acc[i][2 * q], -acc[i][2 * q + 1]);
+  for (int ni = 0; ni < 8; ++ni) {
+    *reinterpret_cast<double2 *>(o + 8 * ni) = make_double2(-acc[ni][0], -acc[ni][1]);
+    *reinterpret_cast<double2 *>(o + 8 * a.ld + 8 * ni) = make_double2(-acc[ni][2], -acc[ni][3]);
   }
 }
 
 // The update of every tile outside the panel columns, persistent: CTA x
-// takes tiles x, x + gridDim.x, ... (row-major over (I, J), J skipping the
-// panel), its chunks one continuous stream through a three-stage ring
-// across tile boundaries (one barrier per chunk: wait for chunk g, barrier,
-// issue chunk g + 2 into the stage chunk g - 1 used, compute chunk g).
-// Warp w computes rows 64 (w / 4) .. + 63 and columns 32 (w % 4) .. + 31 of
-// the tile as 4 x 4 tensor-core tiles of 16 x 8.  A tile's old values are
+// takes tiles x, x + gridDim.x, ... (64 rows x 128 columns, row-major over
+// (I, J), J skipping the panel), its chunks one continuous stream through a
+// two-stage ring across tile boundaries (one barrier per chunk: wait for chunk
+// g, barrier, issue chunk g + 1 into the stage chunk g - 1 used, compute chunk
+// g).  Warp w computes rows 32 (w / 2) .. + 31 and columns 64 (w % 2) .. + 63
+// of the tile as 2 x 8 tensor-core tiles of 16 x 8.  A tile's old values are
 // prefetched into L2 (bulk prefetch, no shared memory) when its first chunk
 // is requested, and read from there in its epilogue.
-__global__ void __launch_bounds__(kGuThreads, 1) gj_update_kernel(const GjArgs a, int tiles) {
+//
+// Two CTAs share an SM, so that one multiplies while the other is in a tile's
+// epilogue (128 KB in and out of L2 after only 128 k of products) or at a
+// barrier: one CTA of 8 warps per SM with tiles of 128 x 128 had the tensor
+// pipe active for 66 % of the time.  All updates of a 9000-row inverse (1.46
+// Tflop): 61.0 ms that way, 56.3 with two CTAs, 51.0 with the copies spread over
+// the products and the epilogue's loads requested ahead (47.4 with no epilogue
+// at all, 41.3 without the copies too).
+__global__ void __launch_bounds__(kGuThreads, 2) gj_update_kernel(const GjArgs a, int tiles) {
   extern __shared__ __align__(16) unsigned char gj_smem[];
-  double *As = reinterpret_cast<double *>(gj_smem);  // [3][128][kGuAS]: W[row][k]
-  double *Bs = As + kGuStages * kGuABuf;              // [3][32][kGuBS]: R[k][col]
+  double *As = reinterpret_cast<double *>(gj_smem);  // [2][64][kGuAS]: W[row][k]
+  double *Bs = As + kGuStages * kGuABuf;              // [2][32][kGuBS]: R[k][col]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
-  const int wr = 64 * (warp >> 2), wc = 32 * (warp & 3);
+  const int wr = 32 * (warp >> 1), wc = 64 * (warp & 1);
   const int ncol = tiles - 1;
-  const int64_t ntile = static_cast<int64_t>(ncol) * tiles;
+  const int64_t ntile = static_cast<int64_t>(ncol) * tiles * (kGjB / kGuM);
   const int64_t first = blockIdx.x;
   if (first >= ntile) return;
   const int mine = static_cast<int>((ntile - first + gridDim.x - 1) / gridDim.x);
@@ -181,118 +188,117 @@ __global__ void __launch_bounds__(kGuThreads, 1) gj_update_kernel(const GjArgs a
   auto tile_rc = [&](int it, int64_t &row0, int64_t &col0) {
     const int64_t tt = first + static_cast<int64_t>(it) * gridDim.x;
     const int I = static_cast<int>(tt / ncol), jx = static_cast<int>(tt % ncol);
-    row0 = static_cast<int64_t>(I) * kGjB;
+    row0 = static_cast<int64_t>(I) * kGuM;
     col0 = static_cast<int64_t>(jx < a.s ? jx : jx + 1) * kGjB;
   };
-  // chunk gc's copies in four parts of 2 + 2 per thread (part p: W
-  // segments u = 2p, 2p + 1 and R segments likewise), so that a chunk's
-  // requests are spread over the compute of the chunk two before it instead
-  // of queueing at the load/store unit all at once; the last part commits
-  auto load_part = [&](int gc, int part) {
-    if (gc < total) {
-      int64_t row0, col0;
-      tile_rc(gc / kGuChunks, row0, col0);
-      const int c = gc % kGuChunks, stage = gc % kGuStages;
-#pragma unroll
-      for (int v = 0; v < 2; ++v) {
-        const int seg = tid + (2 * part + v) * kGuThreads;  // W: 128 rows x 16 segments of 16 B
-        const int m = seg >> 4, q = seg & 15;
-        cp_async16(As + stage * kGuABuf + m * kGuAS + 2 * q, a.A + (row0 + m) * a.ld + k0 + c * kGuKC + 2 * q);
-      }
-#pragma unroll
-      for (int v = 0; v < 2; ++v) {
-        const int seg = tid + (2 * part + v) * kGuThreads;  // R: 32 rows x 64 segments of 16 B
-        const int kk = seg >> 6, q = seg & 63;
-        cp_async16(Bs + stage * kGuBBuf + kk * kGuBS + 2 * q,
-                   a.R + static_cast<int64_t>(c * kGuKC + kk) * a.ld + col0 + 2 * q);
-      }
-      // the tile's old values (none for the pivot block's rows, which become
-      // Q R) on their way into L2
-      if (part == 0 && c == 0 && row0 != k0 && tid < kGjB) {
-        const double *src = a.A + (row0 + tid) * a.ld + col0;
-        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(static_cast<unsigned>(kGjB * sizeof(double)))
-                     : "memory");
-      }
+  // chunk gc's copies: W 64 rows x 16 segments of 16 B (8 a thread), R 32 rows
+  // x 64 segments (16 a thread), issued one or two at a time between the
+  // tensor-core steps of the chunk before (all at once they hold up the
+  // fragments' reads: the load/store unit took 12 % of the kernel's time)
+  const double *lw = nullptr, *lr = nullptr;
+  double *lws = nullptr, *lrs = nullptr;
+  auto load_begin = [&](int gc) {
+    lw = nullptr;
+    if (gc >= total) return;
+    int64_t row0, col0;
+    tile_rc(gc / kGuChunks, row0, col0);
+    const int c = gc % kGuChunks, stage = gc % kGuStages;
+    lw = a.A + (row0 + (tid >> 4)) * a.ld + k0 + c * kGuKC + 2 * (tid & 15);
+    lws = As + stage * kGuABuf + (tid >> 4) * kGuAS + 2 * (tid & 15);
+    lr = a.R + static_cast<int64_t>(c * kGuKC + (tid >> 6)) * a.ld + col0 + 2 * (tid & 63);
+    lrs = Bs + stage * kGuBBuf + (tid >> 6) * kGuBS + 2 * (tid & 63);
+    // the tile's old values (none for the pivot block's rows, which become
+    // Q R) on their way into L2
+    if (c == 0 && (row0 < k0 || row0 >= k0 + kGjB) && tid < kGuM) {
+      const double *src = a.A + (row0 + tid) * a.ld + col0;
+      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(static_cast<unsigned>(kGjB * sizeof(double)))
+                   : "memory");
     }
-    if (part == 3) cp_async_commit();  // an empty group past the end keeps the count uniform
   };
-  auto load = [&](int gc) {
-#pragma unroll
-    for (int part = 0; part < 4; ++part) load_part(gc, part);
+  auto load_w = [&](int v) {
+    if (lw) cp_async16(lws + 8 * v * kGuAS, lw + 8 * v * a.ld);
+  };
+  auto load_r = [&](int v) {
+    if (lw) cp_async16(lrs + 2 * v * kGuBS, lr + 2 * v * a.ld);
   };
 
-  load(0);
-  load(1);
-  double acc[4][4][4];
+  load_begin(0);
 #pragma unroll
-  for (int mi = 0; mi < 4; ++mi)
+  for (int v = 0; v < 8; ++v) load_w(v);
 #pragma unroll
-    for (int ni = 0; ni < 4; ++ni)
+  for (int v = 0; v < 16; ++v) load_r(v);
+  cp_async_commit();
+  double acc[2][8][4];
+#pragma unroll
+  for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+    for (int ni = 0; ni < 8; ++ni)
 #pragma unroll
       for (int i = 0; i < 4; ++i) acc[mi][ni][i] = 0.0;
   for (int gc = 0; gc < total; ++gc) {
-    cp_async_wait<1>();
+    cp_async_wait<0>();
     __syncthreads();
+    load_begin(gc + 1);
     const int stage = gc % kGuStages;
-#pragma unroll
-    for (int ks = 0; ks < kGuKC / 16; ++ks) {
-      const double *as = As + stage * kGuABuf + (wr + g) * kGuAS + 16 * ks + t;
-      const double *bs = Bs + stage * kGuBBuf + (16 * ks + t) * kGuBS + wc + g;
-      double bf[4][4];
-#pragma unroll
-      for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) bf[ni][j] = bs[4 * j * kGuBS + 8 * ni];
-      // A fragments double-buffered: those of row block mi + 1 are read while
-      // the tensor-core steps of row block mi issue
-      double af[2][8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) af[0][i] = as[8 * (i & 1) * kGuAS + 4 * (i >> 1)];
-#pragma unroll
-      for (int mi = 0; mi < 4; ++mi) {
-        if (mi + 1 < 4) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i)
-            af[(mi + 1) & 1][i] = as[(16 * (mi + 1) + 8 * (i & 1)) * kGuAS + 4 * (i >> 1)];
-        }
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni) mma_f64_16816(acc[mi][ni], af[mi & 1], bf[ni]);
-        // chunk gc + 2 into the stage chunk gc - 1 used (free since the barrier)
-        if ((mi & 1) == 1) load_part(gc + 2, 2 * ks + (mi >> 1));
-      }
-    }
-    if (gc % kGuChunks != kGuChunks - 1) continue;
-    // epilogue of tile it: old values (from L2) + W R
+    const bool last = gc % kGuChunks == kGuChunks - 1;
+    // the tile of this chunk: old values (from L2) + W R in its epilogue, a
+    // quarter (8 rows apart, 8 x 2 columns a lane) at a time, the first requested
+    // before the last products and each other one before its predecessor is
+    // stored
     int64_t row0, col0;
     tile_rc(gc / kGuChunks, row0, col0);
-    const bool needC = row0 != k0;
-    double2 old[4][2][4];
+    const bool needC = row0 < k0 || row0 >= k0 + kGjB;
+    double *const o = a.A + (row0 + wr + g) * a.ld + col0 + wc + 2 * t;
+    double2 old[2][8];
+    auto request = [&](int q) {
 #pragma unroll
-    for (int mi = 0; mi < 4; ++mi)
+      for (int ni = 0; ni < 8; ++ni)
+        old[q & 1][ni] = needC ? __ldcg(reinterpret_cast<const double2 *>(o + 8 * q * a.ld + 8 * ni))
+                               : make_double2(0.0, 0.0);
+    };
 #pragma unroll
-      for (int h = 0; h < 2; ++h)
+    for (int ks = 0; ks < kGuKC / 16; ++ks) {
+      if (ks == 1 && last) request(0);
+      const double *as = As + stage * kGuABuf + (wr + g) * kGuAS + 16 * ks + t;
+      const double *bs = Bs + stage * kGuBBuf + (16 * ks + t) * kGuBS + wc + g;
+      double af[2][8];
 #pragma unroll
-        for (int ni = 0; ni < 4; ++ni) {
-          const int r = wr + 16 * mi + g + 8 * h, c = wc + 8 * ni + 2 * t;
-          old[mi][h][ni] = needC ? __ldcg(reinterpret_cast<const double2 *>(a.A + (row0 + r) * a.ld + col0 + c))
-                                 : make_double2(0.0, 0.0);
+      for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) af[mi][i] = as[(16 * mi + 8 * (i & 1)) * kGuAS + 4 * (i >> 1)];
+      // B fragments double-buffered: those of column block ni + 1 are read
+      // while the tensor-core steps of column block ni issue
+      double bf[2][4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) bf[0][j] = bs[4 * j * kGuBS];
+#pragma unroll
+      for (int ni = 0; ni < 8; ++ni) {
+        if (ni + 1 < 8) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) bf[(ni + 1) & 1][j] = bs[4 * j * kGuBS + 8 * (ni + 1)];
         }
 #pragma unroll
-    for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int r = wr + 16 * mi + g + 8 * h;
-        double *o = a.A + (row0 + r) * a.ld + col0;
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni) {
-          const int c = wc + 8 * ni + 2 * t;
-          *reinterpret_cast<double2 *>(o + c) = make_double2(old[mi][h][ni].x + acc[mi][ni][2 * h],
-                                                             old[mi][h][ni].y + acc[mi][ni][2 * h + 1]);
-          acc[mi][ni][2 * h] = 0.0;
-          acc[mi][ni][2 * h + 1] = 0.0;
-        }
+        for (int mi = 0; mi < 2; ++mi) mma_f64_16816(acc[mi][ni], af[mi], bf[ni & 1]);
+        load_r(8 * ks + ni);
+        if (ks == 0) load_w(ni);
       }
+    }
+    cp_async_commit();  // an empty group past the end
+    if (!last) continue;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (q + 1 < 4) request(q + 1);
+#pragma unroll
+      for (int ni = 0; ni < 8; ++ni) {
+        double *c = &acc[q >> 1][ni][2 * (q & 1)];
+        *reinterpret_cast<double2 *>(o + 8 * q * a.ld + 8 * ni) =
+            make_double2(old[q & 1][ni].x + c[0], old[q & 1][ni].y + c[1]);
+        c[0] = 0.0;
+        c[1] = 0.0;
+      }
+    }
   }
+  cp_async_wait<0>();
 }
 
 // The padding of an n x n matrix to np x np: identity (its inverse is the
@@ -381,8 +387,8 @@ int f3d_dense_inverse(double *A, int64_t n, int64_t ld, void *workspace, size_t 
       cudaFuncSetAttribute(gj_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            static_cast<int>(kGjSmemUpdate)) != cudaSuccess)
     return F3D_ERR_CUDA;
-  const int64_t update_tiles = (tiles - 1) * tiles;
-  const unsigned update_grid = static_cast<unsigned>(std::min<int64_t>(update_tiles, sm_count()));
+  const int64_t update_tiles = (tiles - 1) * tiles * (kGjB / kGuM);
+  const unsigned update_grid = static_cast<unsigned>(std::min<int64_t>(update_tiles, 2 * static_cast<int64_t>(sm_count())));
   const int prep_blocks = static_cast<int>(std::min<int64_t>(4 * sm_count(), std::max<int64_t>(1, (np - n) * 2 * np / 256 + 1)));
   gj_prepare_kernel<<<prep_blocks, 256, 0, st>>>(A, n, np, ld, off, size, info, static_cast<int>(tiles));
   if (launch_status()) return F3D_ERR_CUDA;
@@ -394,18 +400,12 @@ int f3d_dense_inverse(double *A, int64_t n, int64_t ld, void *workspace, size_t 
   a.ld = ld;
   a.err = device_error_word();
   if (!a.err) return F3D_ERR_CUDA;
-  const size_t row_bytes = static_cast<size_t>(ld) * sizeof(double);
   for (int s = 0; s < tiles; ++s) {
     const int64_t k0 = static_cast<int64_t>(s) * kGjB;
-    if (cudaMemcpy2DAsync(Q, kGjB * sizeof(double), A + k0 * ld + k0, row_bytes, kGjB * sizeof(double), kGjB,
-                          cudaMemcpyDeviceToDevice, st) != cudaSuccess)
-      return F3D_ERR_CUDA;
-    int rc = f3d_batched_inverse(Q, off, size, 1, kGjB, nullptr, info + s, st);
+    int rc = pivot_block_inverse(A + k0 * ld + k0, ld, Q, off, size, info + s, st);
     if (rc) return rc;
-    if (cudaMemcpyAsync(R, A + k0 * ld, kGjB * row_bytes, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
-      return F3D_ERR_CUDA;
     a.s = s;
-    gj_panel_kernel<<<static_cast<unsigned>(tiles), kGjThreads, kGjSmemPanel, st>>>(a);
+    gj_panel_kernel<<<static_cast<unsigned>(tiles * (kGjB / kGpM)), kGpThreads, kGjSmemPanel, st>>>(a);
     if (launch_status()) return F3D_ERR_CUDA;
     if (tiles > 1) {
       gj_update_kernel<<<update_grid, kGuThreads, kGjSmemUpdate, st>>>(a, static_cast<int>(tiles));

@@ -274,9 +274,9 @@ struct TcInv {
 
 template <int NMAX>
 __global__ void __launch_bounds__(256, NMAX == 64 ? 4 : (NMAX == 96 ? 2 : 1))
-    batched_inverse_tc_kernel(double *__restrict__ A, const int64_t *__restrict__ moff,
-                              const int32_t *__restrict__ sizes, int count, float *__restrict__ A32,
-                              int32_t *__restrict__ info) {
+    batched_inverse_tc_kernel(double *A, const int64_t *__restrict__ moff, const int32_t *__restrict__ sizes,
+                              int count, float *__restrict__ A32, int32_t *__restrict__ info, const double *src,
+                              int64_t src_ld) {
   using T = TcInv<NMAX>;
   constexpr int S = T::kS;
   extern __shared__ __align__(16) unsigned char tc_smem[];
@@ -295,16 +295,19 @@ __global__ void __launch_bounds__(256, NMAX == 64 ? 4 : (NMAX == 96 ? 2 : 1))
   if (n <= 0 || n > NMAX) return;
   double *M = A + moff[b];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (n == NMAX && (reinterpret_cast<uintptr_t>(M) & 15) == 0) {
+  // (src: the block is read from there, row stride src_ld, instead of in place)
+  const double *from = src ? src : M;
+  const int64_t ldm = src ? src_ld : n;
+  if (n == NMAX && (ldm & 1) == 0 && (reinterpret_cast<uintptr_t>(from) & 15) == 0) {
     for (int e = tid; e < NMAX * NMAX / 2; e += T::kThreads)
-      cp_async16(&X[e / (NMAX / 2) * S + 2 * (e % (NMAX / 2))], M + 2 * e);
+      cp_async16(&X[e / (NMAX / 2) * S + 2 * (e % (NMAX / 2))], from + e / (NMAX / 2) * ldm + 2 * (e % (NMAX / 2)));
     cp_async_commit();
     cp_async_wait<0>();
   } else {
 #pragma unroll 4
     for (int e = tid; e < NMAX * NMAX; e += T::kThreads) {
       const int r = e / NMAX, c = e % NMAX;
-      X[r * S + c] = (r < n && c < n) ? M[static_cast<int64_t>(r) * n + c] : (r == c ? 1.0 : 0.0);
+      X[r * S + c] = (r < n && c < n) ? from[r * ldm + c] : (r == c ? 1.0 : 0.0);
     }
   }
   for (int r = tid; r < NMAX; r += T::kThreads) s_step[r] = -16;
@@ -535,6 +538,20 @@ __global__ void __launch_bounds__(128) block_gemv_kernel(const T *__restrict__ M
 
 }  // namespace f3d
 
+namespace f3d {
+// Q (128 x 128, packed) = inverse of the 128 x 128 block at src, row stride
+// ld; off = {0} and size = {128} on the device.
+int pivot_block_inverse(const double *src, int64_t ld, double *Q, const int64_t *off, const int32_t *size,
+                        int32_t *info, cudaStream_t st) {
+  using T = TcInv<128>;
+  if (cudaFuncSetAttribute(batched_inverse_tc_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           static_cast<int>(T::kSmem)) != cudaSuccess)
+    return F3D_ERR_CUDA;
+  batched_inverse_tc_kernel<128><<<1, T::kThreads, T::kSmem, st>>>(Q, off, size, 1, nullptr, info, src, ld);
+  return launch_status();
+}
+}  // namespace f3d
+
 extern "C" {
 
 int f3d_batched_inverse(double *A, const int64_t *matrix_offsets, const int32_t *sizes,
@@ -553,21 +570,21 @@ int f3d_batched_inverse(double *A, const int64_t *matrix_offsets, const int32_t 
                              static_cast<int>(T::kSmem)) != cudaSuccess)
       return F3D_ERR_CUDA;
     f3d::batched_inverse_tc_kernel<64><<<count, T::kThreads, T::kSmem, st>>>(A, matrix_offsets, sizes, count, A32,
-                                                                             info);
+                                                                             info, nullptr, 0);
   } else if (max_n <= 96) {
     using T = f3d::TcInv<96>;
     if (cudaFuncSetAttribute(f3d::batched_inverse_tc_kernel<96>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(T::kSmem)) != cudaSuccess)
       return F3D_ERR_CUDA;
     f3d::batched_inverse_tc_kernel<96><<<count, T::kThreads, T::kSmem, st>>>(A, matrix_offsets, sizes, count, A32,
-                                                                             info);
+                                                                             info, nullptr, 0);
   } else {
     using T = f3d::TcInv<128>;
     if (cudaFuncSetAttribute(f3d::batched_inverse_tc_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(T::kSmem)) != cudaSuccess)
       return F3D_ERR_CUDA;
     f3d::batched_inverse_tc_kernel<128><<<count, T::kThreads, T::kSmem, st>>>(A, matrix_offsets, sizes, count,
-                                                                              A32, info);
+                                                                              A32, info, nullptr, 0);
   }
   return f3d::launch_status();
 }
