@@ -15,8 +15,9 @@
 // (the old block row): every column J outside b becomes
 //   A_.J <- [rows outside b] A_.J + W R_.J
 // one FP64 GEMM of rank 128.  Pivoting is local: Q comes from the batched
-// Gauss-Jordan inverse with partial pivoting inside the 128 x 128 block
-// (f3d_batched_inverse), there is no row exchange across blocks.  Block
+// inverse's Gauss-Jordan kernel with partial pivoting inside the 128 x 128
+// block, which reads the block where it stands (pivot_block_inverse); there
+// is no row exchange across blocks.  Block
 // elimination without global pivoting is stable for the operators this
 // library inverts (second-kind boundary integral operators, whose diagonal
 // blocks carry the 1/w-scaled identity): on spheres of 1000 and 2000 nodes
