@@ -248,11 +248,12 @@ __global__ void __launch_bounds__(kLuThreads) batched_lu_factor_kernel(const LuA
 // 256 threads, 80 registers and at most 79 KB per CTA leave three blocks per
 // SM, whose pivot chains overlap.  (128 threads with two rows each: 1.95 ms
 // on the blocks below; every thread scanning the warps' keys and forming the
-// pivot's reciprocal after the barrier: 1.54 ms.)  Measured on 2000 blocks of
-// 64-256 rows (7.2 Gflop): 1.37 ms, against 5.95 ms for the kernel below
-// with its default panel of 32, 2.38 ms with 16 and 3.19 ms with 8; on 2000
-// blocks of 128 rows 0.67 ms against 1.54 ms (16).  One block of 256 rows
-// alone takes 0.30 ms, 0.99 ms before.
+// pivot's reciprocal after the barrier: 1.54 ms; 64-bit keys posted in three
+// words: 1.37 ms.)  Measured on 2000 blocks of 64-256 rows (7.2 Gflop):
+// 1.34 ms, against 5.95 ms for the kernel below with its default panel of 32,
+// 2.38 ms with 16 and 3.18 ms with 8; on 2000 blocks of 128 rows 0.64 ms
+// against 1.53 ms (16).  One block of 256 rows alone takes 0.30 ms, 0.99 ms
+// before.
 constexpr int kLtThreads = 256;
 constexpr int kLtWarps = kLtThreads / 32;
 constexpr int kLtNB = 16;
@@ -268,10 +269,9 @@ static size_t lt_smem(int max_n) {
 
 struct LtShared {
   __align__(16) double cand[2][kLtWarps][kLtNB];  // each warp's best row, by step parity
-  double rcp[2][kLtWarps];                        // the reciprocal of its candidate
-  unsigned hi[2][kLtWarps], lo[2][kLtWarps];      // the candidate's key
+  uint4 post[2][kLtWarps];                        // its candidate's trailing word, position, and reciprocal
+  unsigned hi[2][kLtWarps];                       // the candidate's key
   __align__(16) double l11[kLtNB][kLtNB];         // column-major unit lower triangle of the panel
-  int pos[2][kLtWarps];
   int piv[kLtNB];
   int phys[kLtMax];
   int info, item;
@@ -317,18 +317,18 @@ __device__ __forceinline__ void lt_factor_one(double *__restrict__ A, int n, int
         if (jj >= nb) break;
         const int par = jj & 1;
         // this thread's candidate: 0 none, 1 a NaN (chosen only if every
-        // candidate is one), else the bits of |a| plus 2
-        const double mag = fabs(v[jj]);
-        const unsigned long long key =
-            done ? 0ull : (mag != mag ? 1ull : static_cast<unsigned long long>(__double_as_longlong(mag)) + 2ull);
+        // candidate is one), else the leading word of |a| plus 2
+        const unsigned mag = static_cast<unsigned>(__double2hiint(v[jj])) & 0x7fffffffu;
+        const bool nan = v[jj] != v[jj];
+        const unsigned hi = done ? 0u : (nan ? 1u : mag + 2u), lo = nan ? 0u : __double2loint(v[jj]);
         // the candidate's reciprocal, beside the search (no branch whatever the
         // row holds): l = v / d is formed from it with one residual correction
         // (Markstein); pivots near the ends of the range divide instead
         const double rcp = reciprocal(v[jj]);
-        const unsigned hi = static_cast<unsigned>(key >> 32), lo = static_cast<unsigned>(key);
         const unsigned hmax = __reduce_max_sync(0xffffffffu, hi);
         bool best = hi == hmax;
-        if (__popc(__ballot_sync(0xffffffffu, best)) > 1) {
+        const unsigned all = __ballot_sync(0xffffffffu, best);
+        if (all & (all - 1u)) {  // equal leading words: the trailing ones, then the position
           const unsigned lmax = __reduce_max_sync(0xffffffffu, best ? lo : 0u);
           best = best && lo == lmax;
           const int pmin = __reduce_min_sync(0xffffffffu, best ? pos : INT_MAX);
@@ -336,9 +336,8 @@ __device__ __forceinline__ void lt_factor_one(double *__restrict__ A, int n, int
         }
         if (best) {  // one lane (a warp with no candidate left posts key 0, which never wins)
           S.hi[par][warp] = hi;
-          S.lo[par][warp] = lo;
-          S.pos[par][warp] = pos;
-          S.rcp[par][warp] = rcp;
+          S.post[par][warp] = make_uint4(lo, static_cast<unsigned>(pos), static_cast<unsigned>(__double2loint(rcp)),
+                                         static_cast<unsigned>(__double2hiint(rcp)));
 #pragma unroll
           for (int j = jj & ~1; j < kLtNB; j += 2)
             *reinterpret_cast<double2 *>(&S.cand[par][warp][j]) = make_double2(v[j], v[j + 1]);
@@ -351,12 +350,13 @@ __device__ __forceinline__ void lt_factor_one(double *__restrict__ A, int n, int
         int bw = __ffs(ties) - 1;
         while (ties &= ties - 1u) {  // equal leading words: the rest of the key, then the position
           const int w = __ffs(ties) - 1;
-          const unsigned lw = S.lo[par][w], lb = S.lo[par][bw];
-          if (lw > lb || (lw == lb && S.pos[par][w] < S.pos[par][bw])) bw = w;
+          const uint4 pw = S.post[par][w], pb = S.post[par][bw];
+          if (pw.x > pb.x || (pw.x == pb.x && static_cast<int>(pw.y) < static_cast<int>(pb.y))) bw = w;
         }
-        const int pp = S.pos[par][bw];
+        const uint4 post = S.post[par][bw];
+        const int pp = static_cast<int>(post.y);
         const double *prow = S.cand[par][bw];
-        const double d = prow[jj], rd = S.rcp[par][bw];
+        const double d = prow[jj], rd = __hiloint2double(static_cast<int>(post.w), static_cast<int>(post.z));
         const bool plain = fabs(d) >= 1e-290 && fabs(d) <= 1e290;
         const int k = k0 + jj;
         if (tid == 0) {

@@ -568,9 +568,10 @@ __global__ void __launch_bounds__(kGeoThreads) quad_geometry_kernel(const double
 // Gauss-Jordan, which needs no back substitution): these systems have
 // condition numbers near 1e17, and on a 200-node sphere of radius 0.5 that
 // moved the weights by 7e-8.
-// 24500 triangles: 7.2 ms (7.7 without the look-ahead and with quotients on
-// the chain of back substitution), against 27.9 ms for unblocked Gauss-Jordan with the
-// matrix in the registers of one CTA per SM, two barriers per pivot.
+// 24500 triangles: 6.9 ms (7.2 with 64-bit keys posted in three words; 7.7
+// also without the look-ahead and with quotients on the chain of back
+// substitution), against 27.9 ms for unblocked Gauss-Jordan with the matrix in
+// the registers of one CTA per SM, two barriers per pivot.
 constexpr int kTriThreads = 256;
 constexpr int kTriWarps = kTriThreads / 32;
 constexpr int kTriS = kQuadDim + 2;  // row stride: 116 columns, the right-hand side, one of padding
@@ -580,11 +581,9 @@ constexpr size_t kTriSmem = static_cast<size_t>(kQuadDim) * kTriS * sizeof(doubl
 struct TriShared {
   __align__(16) double cand[2][kTriPW][16];  // each warp's best row, by step parity
   __align__(16) double l11[16][16];          // column-major unit lower triangle of the panel
-  double rcp[2][kTriPW];                     // the reciprocal of its candidate
+  uint4 post[2][kTriPW];                     // its candidate's trailing word, position, and reciprocal
   double c[kQuadNbr][2];                     // projected centres; then the unknowns
   __align__(16) unsigned hi[2][kTriPW];      // the candidate's key
-  unsigned lo[2][kTriPW];
-  int pos[2][kTriPW];
   int phys[2][kQuadDim];                     // row at each position still to be reduced, by panel parity
   int fin[kQuadDim];                         // row of each pivot
 };
@@ -603,15 +602,15 @@ template <int jj>
 __device__ __forceinline__ void tri_pivot(double (&v)[16], TriShared &S, int k, bool &done, int &pos, int lane,
                                           int warp, int *err) {
   constexpr int par = jj & 1;
-  // this row's candidacy: 0 none, 1 a NaN, else the bits of |a| plus 2
-  const double mag = fabs(v[jj]);
-  const unsigned long long key =
-      done ? 0ull : (mag != mag ? 1ull : static_cast<unsigned long long>(__double_as_longlong(mag)) + 2ull);
+  // this row's candidacy: 0 none, 1 a NaN, else the leading word of |a| plus 2
+  const unsigned mag = static_cast<unsigned>(__double2hiint(v[jj])) & 0x7fffffffu;
+  const bool nan = v[jj] != v[jj];
+  const unsigned hi = done ? 0u : (nan ? 1u : mag + 2u), lo = nan ? 0u : __double2loint(v[jj]);
   const double rcp = 1.0 / v[jj];  // beside the search
-  const unsigned hi = static_cast<unsigned>(key >> 32), lo = static_cast<unsigned>(key);
   const unsigned hmax = __reduce_max_sync(0xffffffffu, hi);
   bool best = hi == hmax;
-  if (__popc(__ballot_sync(0xffffffffu, best)) > 1) {
+  const unsigned all = __ballot_sync(0xffffffffu, best);
+  if (all & (all - 1u)) {  // equal leading words: the trailing ones, then the position
     const unsigned lmax = __reduce_max_sync(0xffffffffu, best ? lo : 0u);
     best = best && lo == lmax;
     const int pmin = __reduce_min_sync(0xffffffffu, best ? pos : INT_MAX);
@@ -619,9 +618,8 @@ __device__ __forceinline__ void tri_pivot(double (&v)[16], TriShared &S, int k, 
   }
   if (best) {  // one lane (a warp with no candidate left posts key 0, which never wins)
     S.hi[par][warp] = hi;
-    S.lo[par][warp] = lo;
-    S.pos[par][warp] = pos;
-    S.rcp[par][warp] = rcp;
+    S.post[par][warp] = make_uint4(lo, static_cast<unsigned>(pos), static_cast<unsigned>(__double2loint(rcp)),
+                                   static_cast<unsigned>(__double2hiint(rcp)));
 #pragma unroll
     for (int j = jj & ~1; j < 16; j += 2)
       *reinterpret_cast<double2 *>(&S.cand[par][warp][j]) = make_double2(v[j], v[j + 1]);
@@ -635,13 +633,14 @@ __device__ __forceinline__ void tri_pivot(double (&v)[16], TriShared &S, int k, 
     // equal leading words: the rest of the key, then the position
     for (int w = bw + 1; w < kTriPW; ++w) {
       if (S.hi[par][w] != top) continue;
-      const unsigned lw = S.lo[par][w], lb = S.lo[par][bw];
-      if (lw > lb || (lw == lb && S.pos[par][w] < S.pos[par][bw])) bw = w;
+      const uint4 pw = S.post[par][w], pb = S.post[par][bw];
+      if (pw.x > pb.x || (pw.x == pb.x && static_cast<int>(pw.y) < static_cast<int>(pb.y))) bw = w;
     }
   }
-  const int pp = S.pos[par][bw];
+  const uint4 post = S.post[par][bw];
+  const int pp = static_cast<int>(post.y);
   const double *prow = S.cand[par][bw];
-  const double d = prow[jj], rd = S.rcp[par][bw];
+  const double d = prow[jj], rd = __hiloint2double(static_cast<int>(post.w), static_cast<int>(post.z));
   if (pos == pp) {  // the pivot row
     pos = k;
     done = true;
