@@ -611,6 +611,28 @@ __device__ __forceinline__ int source_slot(const GemmOp &op, int oct, int slot, 
   return op.table[morton(ix, iy, iz)];
 }
 
+// acc += a chunk's products for the column groups N0 .. N1 - 1 of a warp's two
+template <int N0, int N1>
+__device__ __forceinline__ void products(double (&acc)[3][2][4], const double (*As)[GAS], const double (*Xs)[GXS],
+                                         int t4, int lg, int wc) {
+#pragma unroll
+  for (int ks = 0; ks < GBK; ks += 16) {
+    double bf[2][4];
+#pragma unroll
+    for (int ni = N0; ni < N1; ++ni)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) bf[ni][j] = Xs[ks + t4 + 4 * j][wc + 32 * ni + lg];
+#pragma unroll
+    for (int mi = 0; mi < 3; ++mi) {
+      double af[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) af[q] = As[ks + t4 + 4 * (q >> 1)][16 * mi + lg + 8 * (q & 1)];
+#pragma unroll
+      for (int ni = N0; ni < N1; ++ni) mma_f64_16816(acc[mi][ni], af, bf[ni]);
+    }
+  }
+}
+
 // The chunks (32 k) of all the terms of an item (48 rows x 64 columns of one
 // split) form one stream through two buffers: while chunk i is multiplied,
 // chunk i + 1's densities arrive by cp.async and its kernel values are formed,
@@ -627,9 +649,16 @@ __device__ __forceinline__ int source_slot(const GemmOp &op, int oct, int slot, 
 // 16 k with the gather's addresses formed for each value, 270 with a pointer per
 // column moved on; and 32 k per barrier instead of 16.  All launches of an
 // evaluation at 1e5 points of each kind, order 8: 12.7 ms before, 12.3 (even
-// items), 10.7 (pointers), 9.9 (32 k); at 1e6 70.0 before, 54.2 ms.  The order of
-// every sum is as it was: at order 8 the check-to-equivalent maps turn a
-// rounding there into 1e-8 of the result.
+// items), 10.7 (pointers), 9.9 (32 k); at 1e6 70.0 before, 54.2 ms.  Then a
+// chunk's products in one straight piece of code for each case of live column
+// groups, where a test before each product kept the operands' reads from
+// running ahead (9.35 and 51.7 ms); and the warps' column groups: w and w + 4,
+// not 2 w and 2 w + 1, so that the outer boxes of a tile, which lack sources
+// most often, and a short tile's columns spread over the SM's four quarters,
+// each with a tensor core of its own (8.95 and 49.4 ms).  (Operands read 16
+// bytes at a time: 11.3 and 63.3 ms.)  The order of every sum is as it was: at
+// order 8 the check-to-equivalent maps turn a rounding there into 1e-8 of the
+// result.
 __global__ void __launch_bounds__(GTHREADS, 3) fmm_gemm_kernel(const __grid_constant__ GemmOp op, int rtiles,
                                                                int ctiles) {
   extern __shared__ __align__(16) double g_smem[];
@@ -639,12 +668,12 @@ __global__ void __launch_bounds__(GTHREADS, 3) fmm_gemm_kernel(const __grid_cons
   __shared__ unsigned s_live[2][2];    // its columns that have one
   const int tid = threadIdx.x;
   const int tps = (op.nterms + op.nsplit - 1) / op.nsplit;
-  // FP64 tensor cores (mma.sync m16n8k16): warp w computes columns 16 w .. + 15
-  // of the tile as 3 x 2 tiles of 16 x 8; lane = 4 lg + t4 holds rows lg,
+  // FP64 tensor cores (mma.sync m16n8k16): warp w computes columns 8 w .. + 7 and
+  // 8 w + 32 .. + 39 of the tile as 3 x 2 tiles of 16 x 8; lane = 4 lg + t4 holds rows lg,
   // lg + 8 and columns 2 t4, 2 t4 + 1 of each
   const int lane = tid & 31, warp = tid >> 5;
   const int lg = lane >> 2, t4 = lane & 3;
-  const int wc = 16 * warp;
+  const int wc = 8 * warp;
   // kernel values: one check point and one of a chunk's eight equivalent points per thread
   const int gi = tid % (GBM / 3), ge = tid / (GBM / 3);
   const int chunks = (op.K + GBK - 1) / GBK;
@@ -780,7 +809,7 @@ __global__ void __launch_bounds__(GTHREADS, 3) fmm_gemm_kernel(const __grid_cons
       // the chunk about to be multiplied
       if (pt != cur_t) {
         cur_t = pt;
-        live = s_live[pbuf][warp >> 1] >> (16 * (warp & 1));
+        live = (s_live[pbuf][0] >> (8 * warp) & 255u) | (s_live[pbuf][1] >> (8 * warp) & 255u) << 8;
       }
       asm volatile("cp.async.wait_group 0;" ::: "memory");
       __syncthreads();
@@ -788,29 +817,21 @@ __global__ void __launch_bounds__(GTHREADS, 3) fmm_gemm_kernel(const __grid_cons
       // is overwritten before its term's last chunk is produced)
       if (++pk == chunks) more = next_term();
       if (more) produce(buf ^ 1);
-#pragma unroll
-      for (int ks = 0; ks < GBK; ks += 16) {
-        double bf[2][4];
-#pragma unroll
-        for (int ni = 0; ni < 2; ++ni)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) bf[ni][j] = Xs[buf][ks + t4 + 4 * j][wc + 8 * ni + lg];
-#pragma unroll
-        for (int mi = 0; mi < 3; ++mi) {
-          double af[8];
-#pragma unroll
-          for (int q = 0; q < 8; ++q) af[q] = As[buf][ks + t4 + 4 * (q >> 1)][16 * mi + lg + 8 * (q & 1)];
-#pragma unroll
-          for (int ni = 0; ni < 2; ++ni)
-            if ((live >> (8 * ni)) & 255u) mma_f64_16816(acc[mi][ni], af, bf[ni]);
-        }
-      }
+      // (straight code for each case: a branch inside keeps the operands' reads
+      // from running ahead of the products)
+      const bool l0 = live & 255u, l1 = (live >> 8) & 255u;
+      if (l0 && l1)
+        products<0, 2>(acc, As[buf], Xs[buf], t4, lg, wc);
+      else if (l0)
+        products<0, 1>(acc, As[buf], Xs[buf], t4, lg, wc);
+      else if (l1)
+        products<1, 2>(acc, As[buf], Xs[buf], t4, lg, wc);
     }
 #pragma unroll
     for (int ni = 0; ni < 2; ++ni)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const int col = col0 + wc + 8 * ni + 2 * t4 + e;
+        const int col = col0 + wc + 32 * ni + 2 * t4 + e;
         if (col >= col_end) continue;
         const int slot = op.cols ? op.cols[col] : col;
         double *y = op.nsplit > 1 ? op.partial + (static_cast<int64_t>(split) * op.nslots + slot) * op.ldy
