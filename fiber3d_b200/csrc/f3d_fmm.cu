@@ -297,8 +297,14 @@ __global__ void leaf_ranges_kernel(const uint64_t *__restrict__ kv, int64_t n, i
 // coordinate order within one, so that runs of eight columns near a face of the
 // domain lack the same terms of the interaction list (18 % of the products left
 // out at 8^3 and 17 % at 16^3 leaves; grouping by faces first leaves out 27 % and
-// 23 % but no time: the warps of a tile wait for the one with the most)
-__global__ void octant_keys_kernel(const int *__restrict__ keys, int nbox, int64_t n2, uint64_t *kv,
+// 23 % but no time: the warps of a tile wait for the one with the most).
+// At level 2, where one tile takes all boxes and a term has sources for ten of
+// 64 on average, the eight children of a parent stand together and parents in
+// the order 0 1 2 3 7 6 5 4: then the column groups w and w + 4 of a warp are
+// opposite corners of the domain, of which a term (distance two or more along
+// some axis) reaches at most one.  Half of the products of the order by octant
+// are left and never two groups for one warp: 1.47 ms -> 1.03 at order 8.
+__global__ void octant_keys_kernel(const int *__restrict__ keys, int nbox, int64_t n2, int level, uint64_t *kv,
                                    unsigned *oct_count) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n2) return;
@@ -309,8 +315,12 @@ __global__ void octant_keys_kernel(const int *__restrict__ keys, int nbox, int64
   const unsigned oct = static_cast<unsigned>(keys[i]) & 7u;
   int ix, iy, iz;
   unmorton(static_cast<uint32_t>(keys[i]), ix, iy, iz);
-  const uint64_t at = static_cast<uint64_t>((ix << 16) | (iy << 8) | iz);
-  kv[i] = (static_cast<uint64_t>(oct) << 56) | (at << 32) | static_cast<uint32_t>(i);
+  uint64_t at = static_cast<uint64_t>(oct) << 24 | static_cast<uint64_t>((ix << 16) | (iy << 8) | iz);
+  if (level == 2) {
+    const unsigned parent = static_cast<unsigned>(keys[i]) >> 3;
+    at = ((parent < 4 ? parent : 11 - parent) << 3) | oct;
+  }
+  kv[i] = (at << 32) | static_cast<uint32_t>(i);
   atomicAdd(&oct_count[oct], 1u);
 }
 
@@ -1322,7 +1332,7 @@ int build_tree(f3d_fmm *h, cudaStream_t st) {
     if ((rc = reserve(lv.trg_cols, static_cast<size_t>(lv.ntrg) * sizeof(int)))) return rc;
     unsigned *oc = as<unsigned>(h->scalars) + 32;
     if (cudaMemsetAsync(oc, 0, 8 * sizeof(unsigned), st) != cudaSuccess) return F3D_ERR_CUDA;
-    octant_keys_kernel<<<blocks(n2), 256, 0, st>>>(as<int>(lv.trg_keys), lv.ntrg, n2, as<uint64_t>(h->okv), oc);
+    octant_keys_kernel<<<blocks(n2), 256, 0, st>>>(as<int>(lv.trg_keys), lv.ntrg, n2, l, as<uint64_t>(h->okv), oc);
     if ((rc = launch_status())) return rc;
     if ((rc = sort_u64(as<uint64_t>(h->okv), n2, st))) return rc;
     low_words_kernel<<<blocks(lv.ntrg), 256, 0, st>>>(as<uint64_t>(h->okv), lv.ntrg, as<int>(lv.trg_cols));
