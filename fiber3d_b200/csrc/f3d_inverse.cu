@@ -33,6 +33,7 @@
 #include <climits>
 
 #include "f3d_common.cuh"
+#include "f3d_gemv.cuh"
 
 namespace f3d {
 
@@ -488,43 +489,57 @@ __global__ void __launch_bounds__(256, NMAX == 64 ? 4 : (NMAX == 96 ? 2 : 1))
 }
 
 // y_b = M_b x_b for every block b (M row-major n_b x n_b at moff[b], x and y
-// at voff[b]).  One CTA per block, 8 lanes per row (16-byte loads where the
-// block is aligned), FP64 accumulation.
-template <typename T>
-__global__ void __launch_bounds__(128) block_gemv_kernel(const T *__restrict__ M,
-                                                         const int64_t *__restrict__ moff,
-                                                         const int64_t *__restrict__ voff,
-                                                         const int32_t *__restrict__ sizes,
-                                                         int count, const double *__restrict__ x,
-                                                         double *__restrict__ y) {
+// at voff[b]), a CTA per block.  FP64: the block's rows shared out to the warps,
+// which stream them (16-byte copies where the block allows it).
+constexpr int kBlockGemvWarps = 4;
+__global__ void __launch_bounds__(32 * kBlockGemvWarps) block_gemv_kernel(const double *__restrict__ M,
+                                                                          const int64_t *__restrict__ moff,
+                                                                          const int64_t *__restrict__ voff,
+                                                                          const int32_t *__restrict__ sizes, int count,
+                                                                          const double *__restrict__ x,
+                                                                          double *__restrict__ y) {
+  extern __shared__ __align__(16) double gemv_ring[];
+  const int b = blockIdx.x, warp = threadIdx.x >> 5;
+  if (b >= count) return;
+  const int n = sizes[b];
+  const double *Mb = M + moff[b], *xb = x + voff[b];
+  double *yb = y + voff[b], *ring = gemv_ring + warp * kGemvDepth * kGemvStage;
+  const int lo = warp * n / kBlockGemvWarps, hi = (warp + 1) * n / kBlockGemvWarps;
+  if ((reinterpret_cast<uintptr_t>(Mb) & 15) == 0 && n % 2 == 0)
+    gemv_stream_rows<2>(Mb, xb, yb, lo, hi, n, n, ring);
+  else
+    gemv_stream_rows<1>(Mb, xb, yb, lo, hi, n, n, ring);
+}
+
+// The FP32 copy: 8 lanes per row (16-byte loads where the block is aligned),
+// FP64 accumulation.
+__global__ void __launch_bounds__(128) block_gemv_f32_kernel(const float *__restrict__ M,
+                                                             const int64_t *__restrict__ moff,
+                                                             const int64_t *__restrict__ voff,
+                                                             const int32_t *__restrict__ sizes,
+                                                             int count, const double *__restrict__ x,
+                                                             double *__restrict__ y) {
   extern __shared__ __align__(16) double xs[];
   const int b = blockIdx.x;
   if (b >= count) return;
   const int n = sizes[b];
-  const T *Mb = M + moff[b];
+  const float *Mb = M + moff[b];
   const double *xb = x + voff[b];
   for (int i = threadIdx.x; i < n; i += blockDim.x) xs[i] = xb[i];
   __syncthreads();
-  constexpr int kVec = 16 / sizeof(T);
-  const bool vec = ((reinterpret_cast<uintptr_t>(Mb) & 15) == 0) && (n % kVec == 0);
+  const bool vec = ((reinterpret_cast<uintptr_t>(Mb) & 15) == 0) && (n % 4 == 0);
   const int sub = threadIdx.x & 7;          // lane within the row group
   const int grp = threadIdx.x >> 3;         // 16 row groups per CTA
   for (int r = grp; r < n; r += 16) {
-    const T *row = Mb + static_cast<int64_t>(r) * n;
+    const float *row = Mb + static_cast<int64_t>(r) * n;
     double s = 0.0;
     if (vec) {
-      for (int c = sub * kVec; c < n; c += 8 * kVec) {
-        if constexpr (sizeof(T) == 8) {
-          const double2 v = *reinterpret_cast<const double2 *>(row + c);
-          s = fma(v.x, xs[c], s);
-          s = fma(v.y, xs[c + 1], s);
-        } else {
-          const float4 v = *reinterpret_cast<const float4 *>(row + c);
-          s = fma(static_cast<double>(v.x), xs[c], s);
-          s = fma(static_cast<double>(v.y), xs[c + 1], s);
-          s = fma(static_cast<double>(v.z), xs[c + 2], s);
-          s = fma(static_cast<double>(v.w), xs[c + 3], s);
-        }
+      for (int c = sub * 4; c < n; c += 32) {
+        const float4 v = *reinterpret_cast<const float4 *>(row + c);
+        s = fma(static_cast<double>(v.x), xs[c], s);
+        s = fma(static_cast<double>(v.y), xs[c + 1], s);
+        s = fma(static_cast<double>(v.z), xs[c + 2], s);
+        s = fma(static_cast<double>(v.w), xs[c + 3], s);
       }
     } else {
       for (int c = sub; c < n; c += 8) s = fma(static_cast<double>(row[c]), xs[c], s);
@@ -600,10 +615,10 @@ int f3d_block_gemv(int precision, const void *M, const int64_t *matrix_offsets,
   if (smem > 48 * 1024) return F3D_ERR_TOO_LARGE;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (precision == F3D_FP64) {
-    f3d::block_gemv_kernel<double><<<count, 128, smem, st>>>(
+    f3d::block_gemv_kernel<<<count, 32 * f3d::kBlockGemvWarps, f3d::kBlockGemvWarps * f3d::kGemvWarpSmem, st>>>(
         static_cast<const double *>(M), matrix_offsets, vector_offsets, sizes, count, x, y);
   } else if (precision == F3D_FP32C) {
-    f3d::block_gemv_kernel<float><<<count, 128, smem, st>>>(
+    f3d::block_gemv_f32_kernel<<<count, 128, smem, st>>>(
         static_cast<const float *>(M), matrix_offsets, vector_offsets, sizes, count, x, y);
   } else {
     return F3D_ERR_ARG;

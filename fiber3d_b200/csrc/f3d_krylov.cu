@@ -20,6 +20,7 @@
 #include <type_traits>
 
 #include "f3d_common.cuh"
+#include "f3d_gemv.cuh"
 
 namespace f3d {
 
@@ -165,21 +166,21 @@ __global__ void bump_kernel(int *kptr) {
   if (threadIdx.x == 0 && blockIdx.x == 0) *kptr += 1;
 }
 
-// y = M x, M row-major rows x cols.  Each warp owns kRowsPerWarp rows of a
-// group; x is staged through shared memory in chunks shared by the 32 rows of
+// y = M x, M row-major rows x cols in FP32.  Each warp owns kRowsPerWarp rows of
+// a group; x is staged through shared memory in chunks shared by the 32 rows of
 // the CTA's group, so M streams from HBM once and x mostly from L2.  With
-// VEC > 1 each lane loads VEC consecutive elements (16 bytes) per access; the
-// caller guarantees 16-byte aligned rows (ld and cols multiples of VEC).
-template <typename T, int VEC>
-__device__ __forceinline__ void gemv_rows(const T *__restrict__ M, const double *__restrict__ x, double *y,
-                                          int64_t rows, int64_t cols, int64_t ld, int64_t bx, int64_t gx) {
+// VEC = 4 each lane loads 16 bytes per access; the caller guarantees 16-byte
+// aligned rows (ld and cols multiples of 4).
+template <int VEC>
+__global__ void __launch_bounds__(256) gemv_f32_kernel(const float *__restrict__ M, const double *__restrict__ x,
+                                                       double *y, int64_t rows, int64_t cols, int64_t ld) {
   constexpr int kXChunk = 4096;
   constexpr int kRowsPerWarp = 4;
   __shared__ __align__(16) double xs[kXChunk];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int warps = blockDim.x >> 5;
   const int64_t group = static_cast<int64_t>(warps) * kRowsPerWarp;
-  for (int64_t rb = bx * group; rb < rows; rb += gx * group) {
+  for (int64_t rb = static_cast<int64_t>(blockIdx.x) * group; rb < rows; rb += static_cast<int64_t>(gridDim.x) * group) {
     double acc[kRowsPerWarp];
 #pragma unroll
     for (int q = 0; q < kRowsPerWarp; ++q) acc[q] = 0.0;
@@ -193,20 +194,11 @@ __device__ __forceinline__ void gemv_rows(const T *__restrict__ M, const double 
       for (int q = 0; q < kRowsPerWarp; ++q) {
         const int64_t r = rw + q;
         if (r < rows) {
-          const T *row = M + r * ld + c0;
+          const float *row = M + r * ld + c0;
           double a = acc[q];
           if (VEC == 1) {
 #pragma unroll 4
             for (int i = lane; i < cw; i += 32) a = fma(static_cast<double>(row[i]), xs[i], a);
-          } else if constexpr (sizeof(T) == 8) {
-            const double2 *rv = reinterpret_cast<const double2 *>(row);
-            const int nv = cw / 2;
-#pragma unroll 2
-            for (int i = lane; i < nv; i += 32) {
-              const double2 d = rv[i];
-              a = fma(d.x, xs[2 * i], a);
-              a = fma(d.y, xs[2 * i + 1], a);
-            }
           } else {
             const float4 *rv = reinterpret_cast<const float4 *>(row);
             const int nv = cw / 4;
@@ -234,25 +226,44 @@ __device__ __forceinline__ void gemv_rows(const T *__restrict__ M, const double 
 }
 
 
-template <typename T, int VEC>
-__global__ void __launch_bounds__(256) gemv_kernel(const T *__restrict__ M,
-                                                   const double *__restrict__ x, double *y,
-                                                   int64_t rows, int64_t cols, int64_t ld) {
-  gemv_rows<T, VEC>(M, x, y, rows, cols, ld, blockIdx.x, gridDim.x);
+// y = M x in FP64: an even share of the rows for each warp.
+constexpr int kGemvWarps = 8;
+template <int VEC>
+__global__ void __launch_bounds__(32 * kGemvWarps) gemv_kernel(const double *__restrict__ M,
+                                                               const double *__restrict__ x, double *y, int64_t rows,
+                                                               int64_t cols, int64_t ld) {
+  extern __shared__ __align__(16) double gemv_ring[];
+  const int warp = threadIdx.x >> 5;
+  const int64_t w = static_cast<int64_t>(blockIdx.x) * kGemvWarps + warp;
+  const int64_t nw = static_cast<int64_t>(gridDim.x) * kGemvWarps;
+  gemv_stream_rows<VEC>(M, x, y, w * rows / nw, (w + 1) * rows / nw, cols, ld,
+                        gemv_ring + warp * kGemvDepth * kGemvStage);
 }
 
 // count square FP64 matrices in one launch: matrix b (n[b] x n[b], row-major
 // at M + m_off[b]) times x + x_off[b] into y + y_off[b]; blockIdx.y = b.
 template <int VEC>
-__global__ void __launch_bounds__(256) gemv_batched_kernel(const double *__restrict__ M,
-                                                           const int64_t *__restrict__ m_off,
-                                                           const int64_t *__restrict__ n,
-                                                           const int64_t *__restrict__ x_off,
-                                                           const int64_t *__restrict__ y_off,
-                                                           const double *__restrict__ x, double *y) {
-  const int b = blockIdx.y;
+__global__ void __launch_bounds__(32 * kGemvWarps) gemv_batched_kernel(const double *__restrict__ M,
+                                                                       const int64_t *__restrict__ m_off,
+                                                                       const int64_t *__restrict__ n,
+                                                                       const int64_t *__restrict__ x_off,
+                                                                       const int64_t *__restrict__ y_off,
+                                                                       const double *__restrict__ x, double *y) {
+  extern __shared__ __align__(16) double gemv_ring[];
+  const int b = blockIdx.y, warp = threadIdx.x >> 5;
   const int64_t nb = n[b];
-  gemv_rows<double, VEC>(M + m_off[b], x + x_off[b], y + y_off[b], nb, nb, nb, blockIdx.x, gridDim.x);
+  const int64_t w = static_cast<int64_t>(blockIdx.x) * kGemvWarps + warp;
+  const int64_t nw = static_cast<int64_t>(gridDim.x) * kGemvWarps;
+  gemv_stream_rows<VEC>(M + m_off[b], x + x_off[b], y + y_off[b], w * nb / nw, (w + 1) * nb / nw, nb, nb,
+                        gemv_ring + warp * kGemvDepth * kGemvStage);
+}
+
+constexpr size_t kGemvSmem = kGemvWarps * kGemvWarpSmem;
+
+template <typename K>
+static bool gemv_allow(K kernel) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGemvSmem)) ==
+         cudaSuccess;
 }
 
 // Row r of M (cols entries) -> FP16 row of M16 scaled by row_scale[r] = 2^e,
@@ -560,13 +571,13 @@ int f3d_gemv_batched(const double *M, const int64_t *m_off, const int64_t *n, co
   if (!M || !m_off || !n || !x_off || !y_off || !x || !y) return F3D_ERR_NULL;
   if (vec && reinterpret_cast<uintptr_t>(M) % 16 != 0) return F3D_ERR_ALIGN;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int64_t per = std::max<int64_t>(1, std::min<int64_t>((max_n + 31) / 32,
-                                                             (static_cast<int64_t>(f3d::sm_count()) * 4 + count - 1) / count));
+  // two CTAs per SM in all, at least a row for each warp
+  const int64_t per = std::max<int64_t>(1, std::min<int64_t>((max_n + f3d::kGemvWarps - 1) / f3d::kGemvWarps,
+                                                             (static_cast<int64_t>(f3d::sm_count()) * 2 + count - 1) / count));
   const dim3 grid(static_cast<unsigned>(per), static_cast<unsigned>(count));
-  if (vec)
-    f3d::gemv_batched_kernel<2><<<grid, 256, 0, st>>>(M, m_off, n, x_off, y_off, x, y);
-  else
-    f3d::gemv_batched_kernel<1><<<grid, 256, 0, st>>>(M, m_off, n, x_off, y_off, x, y);
+  auto kernel = vec ? f3d::gemv_batched_kernel<2> : f3d::gemv_batched_kernel<1>;
+  if (!f3d::gemv_allow(kernel)) return F3D_ERR_CUDA;
+  kernel<<<grid, 32 * f3d::kGemvWarps, f3d::kGemvSmem, st>>>(M, m_off, n, x_off, y_off, x, y);
   return f3d::launch_status();
 }
 
@@ -583,16 +594,18 @@ int f3d_gemv(int precision, const void *M, int64_t ld, const double *x, double *
   const uintptr_t base = reinterpret_cast<uintptr_t>(M);
   if (precision == F3D_FP64) {
     const bool vec = (base % 16 == 0) && (ld % 2 == 0) && (cols % 2 == 0);
-    if (vec)
-      f3d::gemv_kernel<double, 2><<<grid, 256, 0, st>>>(static_cast<const double *>(M), x, y, rows, cols, ld);
-    else
-      f3d::gemv_kernel<double, 1><<<grid, 256, 0, st>>>(static_cast<const double *>(M), x, y, rows, cols, ld);
+    const unsigned two_per_sm = static_cast<unsigned>(
+        std::min<int64_t>((rows + f3d::kGemvWarps - 1) / f3d::kGemvWarps, static_cast<int64_t>(f3d::sm_count()) * 2));
+    auto kernel = vec ? f3d::gemv_kernel<2> : f3d::gemv_kernel<1>;
+    if (!f3d::gemv_allow(kernel)) return F3D_ERR_CUDA;
+    kernel<<<two_per_sm, 32 * f3d::kGemvWarps, f3d::kGemvSmem, st>>>(static_cast<const double *>(M), x, y, rows, cols,
+                                                                    ld);
   } else if (precision == F3D_FP32C) {
     const bool vec = (base % 16 == 0) && (ld % 4 == 0) && (cols % 4 == 0);
     if (vec)
-      f3d::gemv_kernel<float, 4><<<grid, 256, 0, st>>>(static_cast<const float *>(M), x, y, rows, cols, ld);
+      f3d::gemv_f32_kernel<4><<<grid, 256, 0, st>>>(static_cast<const float *>(M), x, y, rows, cols, ld);
     else
-      f3d::gemv_kernel<float, 1><<<grid, 256, 0, st>>>(static_cast<const float *>(M), x, y, rows, cols, ld);
+      f3d::gemv_f32_kernel<1><<<grid, 256, 0, st>>>(static_cast<const float *>(M), x, y, rows, cols, ld);
   } else {
     return F3D_ERR_ARG;
   }
