@@ -17,8 +17,11 @@ namespace f3d {
 // 33 and 12 us; 512 blocks of 128 x 128 29 and 15 us.  (Four rows: the same; eight:
 // 5 % slower at 12000; a quarter of the bytes in flight: 20 %.)
 constexpr int kGemvRows = 2, kGemvDepth = 6;
-constexpr int kGemvStage = (kGemvRows + 1) * 64;  // doubles: x and the rows
-constexpr size_t kGemvWarpSmem = static_cast<size_t>(kGemvDepth) * kGemvStage * sizeof(double);
+template <int ROWS = kGemvRows, int DEPTH = kGemvDepth>
+constexpr int gemv_ring_doubles() {
+  return DEPTH * (ROWS + 1) * 64;  // x and the rows
+}
+constexpr size_t kGemvWarpSmem = gemv_ring_doubles() * sizeof(double);
 
 __device__ __forceinline__ void gemv_copy8(double *smem, const double *gmem, bool valid) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_addr(smem)), "l"(gmem), "r"(valid ? 8 : 0)
@@ -29,13 +32,14 @@ __device__ __forceinline__ void gemv_copy16(double *smem, const double *gmem, bo
                : "memory");
 }
 
-// y[r] = M[r] . x for r in [r_lo, r_hi), by one warp; ring: kGemvWarpSmem bytes
+// y[r] = M[r] . x for r in [r_lo, r_hi), by one warp; ring: gemv_ring_doubles
 // of its own, 16-byte aligned.  VEC 2: rows 16-byte aligned and cols even (16-byte
 // copies); VEC 1: any rows.  Columns past the last count as zero times zero.
-template <int VEC>
+template <int VEC, int ROWS = kGemvRows, int DEPTH = kGemvDepth>
 __device__ __forceinline__ void gemv_stream_rows(const double *__restrict__ M, const double *__restrict__ x,
                                                  double *y, int64_t r_lo, int64_t r_hi, int64_t cols, int64_t ld,
                                                  double *ring) {
+  constexpr int kStage = (ROWS + 1) * 64;
   const int lane = threadIdx.x & 31;
   // this lane's two columns of a stage
   const int l0 = VEC == 2 ? 2 * lane : lane, l1 = VEC == 2 ? l0 + 1 : l0 + 32;
@@ -47,11 +51,11 @@ __device__ __forceinline__ void gemv_stream_rows(const double *__restrict__ M, c
     if (pr < r_hi) {
       const int64_t c0 = 64 * ps + l0, c1 = 64 * ps + l1;
       const bool v0 = c0 < cols, v1 = c1 < cols;
-      double *d = ring + pb * kGemvStage;
+      double *d = ring + pb * kStage;
       gemv_copy8(d + l0, v0 ? x + c0 : x, v0);
       gemv_copy8(d + l1, v1 ? x + c1 : x, v1);
 #pragma unroll
-      for (int q = 0; q < kGemvRows; ++q) {
+      for (int q = 0; q < ROWS; ++q) {
         const bool in = pr + q < r_hi;
         const double *row = M + (pr + q) * ld;
         if (VEC == 2) {
@@ -63,33 +67,33 @@ __device__ __forceinline__ void gemv_stream_rows(const double *__restrict__ M, c
       }
       if (++ps == stages) {
         ps = 0;
-        pr += kGemvRows;
+        pr += ROWS;
       }
-      if (++pb == kGemvDepth) pb = 0;
+      if (++pb == DEPTH) pb = 0;
     }
     cp_async_commit();
   };
 #pragma unroll
-  for (int d = 0; d < kGemvDepth - 1; ++d) copy();
+  for (int d = 0; d < DEPTH - 1; ++d) copy();
   int b = 0;
-  for (int64_t r = r_lo; r < r_hi; r += kGemvRows) {
-    double acc[kGemvRows];
+  for (int64_t r = r_lo; r < r_hi; r += ROWS) {
+    double acc[ROWS];
 #pragma unroll
-    for (int q = 0; q < kGemvRows; ++q) acc[q] = 0.0;
+    for (int q = 0; q < ROWS; ++q) acc[q] = 0.0;
     for (int64_t s = 0; s < stages; ++s) {
-      cp_async_wait<kGemvDepth - 2>();
-      const double *d = ring + b * kGemvStage;
+      cp_async_wait<DEPTH - 2>();
+      const double *d = ring + b * kStage;
       const double x0 = d[l0], x1 = d[l1];
 #pragma unroll
-      for (int q = 0; q < kGemvRows; ++q) {
+      for (int q = 0; q < ROWS; ++q) {
         const double *m = d + 64 * (q + 1);
         acc[q] = fma(m[l1], x1, fma(m[l0], x0, acc[q]));
       }
-      if (++b == kGemvDepth) b = 0;
+      if (++b == DEPTH) b = 0;
       copy();  // into the slot read one stage before
     }
 #pragma unroll
-    for (int q = 0; q < kGemvRows; ++q) {
+    for (int q = 0; q < ROWS; ++q) {
       double a = acc[q];
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);

@@ -503,7 +503,7 @@ __global__ void __launch_bounds__(32 * kBlockGemvWarps) block_gemv_kernel(const 
   if (b >= count) return;
   const int n = sizes[b];
   const double *Mb = M + moff[b], *xb = x + voff[b];
-  double *yb = y + voff[b], *ring = gemv_ring + warp * kGemvDepth * kGemvStage;
+  double *yb = y + voff[b], *ring = gemv_ring + warp * gemv_ring_doubles();
   const int lo = warp * n / kBlockGemvWarps, hi = (warp + 1) * n / kBlockGemvWarps;
   if ((reinterpret_cast<uintptr_t>(Mb) & 15) == 0 && n % 2 == 0)
     gemv_stream_rows<2>(Mb, xb, yb, lo, hi, n, n, ring);

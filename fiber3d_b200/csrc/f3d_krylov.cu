@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(32 * kGemvWarps) gemv_kernel(const double *__r
   const int64_t w = static_cast<int64_t>(blockIdx.x) * kGemvWarps + warp;
   const int64_t nw = static_cast<int64_t>(gridDim.x) * kGemvWarps;
   gemv_stream_rows<VEC>(M, x, y, w * rows / nw, (w + 1) * rows / nw, cols, ld,
-                        gemv_ring + warp * kGemvDepth * kGemvStage);
+                        gemv_ring + warp * gemv_ring_doubles());
 }
 
 // count square FP64 matrices in one launch: matrix b (n[b] x n[b], row-major
@@ -255,15 +255,46 @@ __global__ void __launch_bounds__(32 * kGemvWarps) gemv_batched_kernel(const dou
   const int64_t w = static_cast<int64_t>(blockIdx.x) * kGemvWarps + warp;
   const int64_t nw = static_cast<int64_t>(gridDim.x) * kGemvWarps;
   gemv_stream_rows<VEC>(M + m_off[b], x + x_off[b], y + y_off[b], w * nb / nw, (w + 1) * nb / nw, nb, nb,
-                        gemv_ring + warp * kGemvDepth * kGemvStage);
+                        gemv_ring + warp * gemv_ring_doubles());
 }
 
 constexpr size_t kGemvSmem = kGemvWarps * kGemvWarpSmem;
 
 template <typename K>
-static bool gemv_allow(K kernel) {
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGemvSmem)) ==
+static bool gemv_allow(K kernel, size_t smem = kGemvSmem) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) ==
          cudaSuccess;
+}
+
+// The product on a part of each SM, for a stream beside a kernel bound by the
+// FP64 pipe (the pair sums, ten CTAs of 64 threads and 96 registers per SM): one
+// CTA of four warps with 54 KB in rings of eight rows.  What the sum loses is
+// issue slots and shared memory cycles, so fewer instructions a byte count here:
+// with rings of two rows the Oseen sum of 512 fibers beside the product with an
+// 18000 x 18000 inverse takes 743 us (eight warps) or 750 (four), with four rows
+// 695, with eight 678, against 562 alone; the product then takes 595 us instead
+// of 410, and the pair together 700 instead of 970.  (Rows requested as bulk
+// copies: 612 us alone already; loads into registers behind an L2 prefetch: the
+// sum and the product took longer than one after the other.)  The preference for
+// the largest shared memory keeps the sum's CTAs on the SMs the product has
+// taken; without it some ring sizes ran one after the other.
+constexpr int kBesideWarps = 4, kBesideRows = 8, kBesideDepth = 3;
+constexpr size_t kBesideSmem = kBesideWarps * gemv_ring_doubles<kBesideRows, kBesideDepth>() * sizeof(double);
+template <int VEC>
+__global__ void __launch_bounds__(32 * kBesideWarps) gemv_beside_kernel(const double *__restrict__ M,
+                                                                        const double *__restrict__ x, double *y,
+                                                                        int64_t rows, int64_t cols, int64_t ld) {
+  extern __shared__ __align__(16) double gemv_ring[];
+  const int warp = threadIdx.x >> 5;
+  const int64_t w = static_cast<int64_t>(blockIdx.x) * kBesideWarps + warp;
+  const int64_t nw = static_cast<int64_t>(gridDim.x) * kBesideWarps;
+  gemv_stream_rows<VEC, kBesideRows, kBesideDepth>(M, x, y, w * rows / nw, (w + 1) * rows / nw, cols, ld,
+                                                   gemv_ring + warp * gemv_ring_doubles<kBesideRows, kBesideDepth>());
+}
+
+// whether the rows can be copied 16 bytes at a time
+static bool gemv_vec(const double *M, int64_t ld, int64_t cols) {
+  return reinterpret_cast<uintptr_t>(M) % 16 == 0 && ld % 2 == 0 && cols % 2 == 0;
 }
 
 // Row r of M (cols entries) -> FP16 row of M16 scaled by row_scale[r] = 2^e,
@@ -581,6 +612,23 @@ int f3d_gemv_batched(const double *M, const int64_t *m_off, const int64_t *n, co
   return f3d::launch_status();
 }
 
+int f3d_gemv_beside(const double *M, int64_t ld, const double *x, double *y, int64_t rows, int64_t cols,
+                    void *stream) {
+  if (!M || !x || !y) return F3D_ERR_NULL;
+  if (rows < 0 || cols < 0 || ld < cols) return F3D_ERR_SHAPE;
+  if (rows == 0) return F3D_OK;
+  const unsigned grid = static_cast<unsigned>(std::min<int64_t>((rows + f3d::kBesideWarps - 1) / f3d::kBesideWarps,
+                                                                static_cast<int64_t>(f3d::sm_count())));
+  auto kernel = f3d::gemv_vec(M, ld, cols) ? f3d::gemv_beside_kernel<2> : f3d::gemv_beside_kernel<1>;
+  if (!f3d::gemv_allow(kernel, f3d::kBesideSmem) ||
+      cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) !=
+          cudaSuccess)
+    return F3D_ERR_CUDA;
+  kernel<<<grid, 32 * f3d::kBesideWarps, f3d::kBesideSmem, static_cast<cudaStream_t>(stream)>>>(M, x, y, rows, cols,
+                                                                                               ld);
+  return f3d::launch_status();
+}
+
 int f3d_gemv(int precision, const void *M, int64_t ld, const double *x, double *y, int64_t rows,
              int64_t cols, void *stream) {
   if (!M || !x || !y) return F3D_ERR_NULL;
@@ -589,19 +637,17 @@ int f3d_gemv(int precision, const void *M, int64_t ld, const double *x, double *
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const unsigned grid = static_cast<unsigned>(std::max<int64_t>(
       1, std::min<int64_t>((rows + 31) / 32, static_cast<int64_t>(f3d::sm_count()) * 4)));
-  // 16-byte vector loads when every row starts 16-byte aligned and the x
-  // chunks (4096 elements) split into whole vectors.
-  const uintptr_t base = reinterpret_cast<uintptr_t>(M);
   if (precision == F3D_FP64) {
-    const bool vec = (base % 16 == 0) && (ld % 2 == 0) && (cols % 2 == 0);
+    const double *Md = static_cast<const double *>(M);
     const unsigned two_per_sm = static_cast<unsigned>(
         std::min<int64_t>((rows + f3d::kGemvWarps - 1) / f3d::kGemvWarps, static_cast<int64_t>(f3d::sm_count()) * 2));
-    auto kernel = vec ? f3d::gemv_kernel<2> : f3d::gemv_kernel<1>;
+    auto kernel = f3d::gemv_vec(Md, ld, cols) ? f3d::gemv_kernel<2> : f3d::gemv_kernel<1>;
     if (!f3d::gemv_allow(kernel)) return F3D_ERR_CUDA;
-    kernel<<<two_per_sm, 32 * f3d::kGemvWarps, f3d::kGemvSmem, st>>>(static_cast<const double *>(M), x, y, rows, cols,
-                                                                    ld);
+    kernel<<<two_per_sm, 32 * f3d::kGemvWarps, f3d::kGemvSmem, st>>>(Md, x, y, rows, cols, ld);
   } else if (precision == F3D_FP32C) {
-    const bool vec = (base % 16 == 0) && (ld % 4 == 0) && (cols % 4 == 0);
+    // 16-byte vector loads when every row starts 16-byte aligned and the x
+    // chunks (4096 elements) split into whole vectors.
+    const bool vec = reinterpret_cast<uintptr_t>(M) % 16 == 0 && (ld % 4 == 0) && (cols % 4 == 0);
     if (vec)
       f3d::gemv_f32_kernel<4><<<grid, 256, 0, st>>>(static_cast<const float *>(M), x, y, rows, cols, ld);
     else

@@ -102,15 +102,19 @@ class DeviceGMRES:
         _lib.call("f3d_krylov_norm", _lib.ptr(w), w.numel(), None, None, _lib.ptr(beta), _lib.ptr(self.wsn),
                   self.wsn.numel(), st)
 
-    def _arnoldi(self, matvec, pc, aux=None):
+    def _arnoldi(self, matvec, pc, aux=None, pc_matvec=None):
         """One Arnoldi step on the current stream (graph-capturable).  With
         `aux` (a device vector the matvec writes, e.g. its pair sums) its
-        norm after the matvec is recorded for the step."""
+        norm after the matvec is recorded for the step.  `pc_matvec(v, z, w)`
+        does both operators where the system overlaps them."""
         st = _lib.stream_handle(self.device)
         n, ldv = self.n, self.n
-        pc(self.cur, self.z)
+        if pc_matvec is not None:
+            pc_matvec(self.cur, self.z, self.w)
+        else:
+            pc(self.cur, self.z)
+            matvec(self.z, self.w)
         _lib.call("f3d_krylov_store", _lib.ptr(self.z), _lib.ptr(self.k), -1, _lib.ptr(self.Z), n, n, st)
-        matvec(self.z, self.w)
         if aux is not None:
             _lib.call("f3d_krylov_norm", _lib.ptr(aux), aux.numel(), _lib.ptr(self.k), _lib.ptr(self.aux),
                       _lib.ptr(self.auxbeta), _lib.ptr(self.wsn), self.wsn.numel(), st)
@@ -129,11 +133,11 @@ class DeviceGMRES:
         if aux is not None:
             self.h_host[2 * m2:3 * m2].copy_(self.aux, non_blocking=True)
 
-    def _step(self, matvec, pc, key, use_graph, aux=None):
+    def _step(self, matvec, pc, key, use_graph, aux=None, pc_matvec=None):
         if not use_graph:
-            self._arnoldi(matvec, pc, aux)
+            self._arnoldi(matvec, pc, aux, pc_matvec)
             return
-        key = (key, aux is not None)
+        key = (key, aux is not None, pc_matvec is not None)
         g = self.graph.get(key)
         if g is None:
             # warm-up outside capture on a side stream (allocations, lazy init)
@@ -141,13 +145,13 @@ class DeviceGMRES:
             s.wait_stream(torch.cuda.current_stream(self.device))
             with torch.cuda.stream(s):
                 saved = (self.k.clone(), self.cur.clone(), self.V.clone(), self.Z.clone())
-                self._arnoldi(matvec, pc, aux)
+                self._arnoldi(matvec, pc, aux, pc_matvec)
                 self.k.copy_(saved[0]); self.cur.copy_(saved[1]); self.V.copy_(saved[2])
                 self.Z.copy_(saved[3])
             torch.cuda.current_stream(self.device).wait_stream(s)
             g = torch.cuda.CUDAGraph()
             with torch.cuda.graph(g):
-                self._arnoldi(matvec, pc, aux)
+                self._arnoldi(matvec, pc, aux, pc_matvec)
             self.graph[key] = g
         self.graph[key].replay()
 
@@ -170,7 +174,8 @@ class DeviceGMRES:
     # ------------------------------------------------------------- solve ---
     def solve(self, matvec, pc, b: torch.Tensor, x0: torch.Tensor | None = None, rtol=1e-8,
               maxiter=200, use_graph=True, key="default", bnorm=None, verify=True, aux=None,
-              r0: torch.Tensor | None = None, rnorm0: float | None = None, first_step_done: bool = False):
+              r0: torch.Tensor | None = None, rnorm0: float | None = None, first_step_done: bool = False,
+              pc_matvec=None):
         """Solve A x = b with right preconditioner pc = P^-1.
 
         Returns (x, info, iterations, history of relative residual estimates).
@@ -185,6 +190,8 @@ class DeviceGMRES:
         x0 is None) when the caller knows it.  With `first_step_done` the
         caller has already run start_cycle() on that residual and the first
         Arnoldi step (same matvec, pc, key and aux), and passes rnorm0.
+        `pc_matvec(v, z, w)`, where given, does z = P^-1 v and w = A z of an
+        Arnoldi step in one call.
         """
         self.last_aux_sum = 0.0
         n, m = self.n, self.m
@@ -238,7 +245,7 @@ class DeviceGMRES:
             j_done = 0
             for j in range(m):
                 if not (prestarted and j == 0):
-                    self._step(matvec, pc, key, use_graph, aux)
+                    self._step(matvec, pc, key, use_graph, aux, pc_matvec)
                 torch.cuda.current_stream(dev).synchronize()
                 col = (hh[:j + 1] + hh[m2:m2 + j + 1]).tolist()
                 sub = float(hh[j + 1])           # subdiagonal |w|
@@ -311,7 +318,8 @@ def solve_system(system, tol=1e-8, restart=100, maxiter=200, x0=None, mixed=Fals
             torch.sub(b, r0, out=r0)
         x, info, its, hist = g.solve(lambda a, o: system.matvec(a, o, "fp64"),
                                      lambda a, o: system.pc(a, o, "fp64"), b, x0=x0, rtol=tol,
-                                     maxiter=maxiter, use_graph=use_graph, key="fp64", r0=r0)
+                                     maxiter=maxiter, use_graph=use_graph, key="fp64", r0=r0,
+                                     pc_matvec=getattr(system, "pc_matvec", None))
         return {"x": x, "info": info, "iterations": its, "history": hist, "refinements": 0,
                 "seconds": time.perf_counter() - t0}
     # mixed: FP32C inner solves; outer residuals FP32C while the bound holds

@@ -235,15 +235,19 @@ class ShellOperator:
         _lib.call("f3d_quantize_rows_f16", _lib.ptr(self.inv64), ld, m, m, 3, _lib.ptr(self.inv16), m,
                   _lib.ptr(self.scale16), _lib.ptr(self.diag16), _lib.stream_handle(self.device))
 
-    def apply(self, x: torch.Tensor, y: torch.Tensor, storage: str = "fp64") -> torch.Tensor:
+    def apply(self, x: torch.Tensor, y: torch.Tensor, storage: str = "fp64", beside: bool = False) -> torch.Tensor:
         """y = P_shell^-1 x from the FP64, FP32 or FP16 copy of the inverse
-        (pc="block": the 3 x 3 block inverses, in FP64 whatever `storage`)."""
+        (pc="block": the 3 x 3 block inverses, in FP64 whatever `storage`).
+        `beside` (FP64 dense inverse): the product on a part of each SM, for a
+        stream that runs beside a pair sum."""
         m = 3 * self.n
         st = _lib.stream_handle(self.device)
         if self.pc == "block":
             _lib.call("f3d_block3_gemv", _lib.ptr(self.block_inv), _lib.ptr(x), _lib.ptr(y), self.n, st)
             return y
-        if storage == "fp16":
+        if beside and storage == "fp64":
+            _lib.call("f3d_gemv_beside", _lib.ptr(self.inv64), self.ld, _lib.ptr(x), _lib.ptr(y), m, m, st)
+        elif storage == "fp16":
             _lib.call("f3d_gemv_f16", _lib.ptr(self.inv16), m, _lib.ptr(self.scale16), _lib.ptr(self.diag16), 3,
                       _lib.ptr(x), _lib.ptr(y), m, m, st)
         else:
@@ -439,6 +443,7 @@ class HydroSystem:
         self.v2 = torch.zeros(3 * self.ntrg, dtype=torch.float64, device=dev)
         self._pending_x0 = None
         self._dual_ws = None
+        self._side = None  # the stream of the periphery's product in pc_matvec
         self.scratch = torch.zeros(4, dtype=torch.float64, device=dev)
         self.oseen = _PairCall("oseen", "skip_group", self.x_fib, self.trg, self.fw, None, self.src_grp,
                                self.trg_grp, self.v, P.eta, P.reg, P.eps_dist) if nF else None
@@ -705,12 +710,14 @@ class HydroSystem:
 
     # ------------------------------------------------------------------------
     def matvec(self, x: torch.Tensor, y: torch.Tensor, precision: str = "fp64",
-               oseen_done: bool = False) -> torch.Tensor:
+               oseen_done: bool = False, join: torch.cuda.Stream | None = None) -> torch.Tensor:
         """y = A x (tstep.py:1003-1178).  With `oseen_done` the FP64 Oseen
         flow of x's fiber forces is the one update(x) summed (see
         :meth:`pending_oseen`).  precision "split": FP64 pair sums on the
         fiber targets, FP32C stresslet sums on the body and periphery
-        targets (whose rows take the flow with gain 1)."""
+        targets (whose rows take the flow with gain 1).  `join`: a stream that
+        may still be writing the periphery's part of x; it is waited for
+        before anything but the fibers' part is read."""
         st = _lib.stream_handle(self.device)
         nF, nB, nS = self.nF, self.nB, self.nS
         XT = x[self.o_fib:]
@@ -724,6 +731,8 @@ class HydroSystem:
                           _lib.ptr(XT), _lib.ptr(self.fw), nF, 1, st)
                 self.oseen("fp64" if split else precision, accumulate=False)
             first = False
+        if join is not None:
+            torch.cuda.current_stream(self.device).wait_stream(join)
         if self.nstress:
             _lib.call("f3d_gather_segments", _lib.ptr(x), _lib.ptr(self.stress_dens), _lib.ptr(self.seg[0]),
                       _lib.ptr(self.seg[1]), _lib.ptr(self.seg[2]), self.seg[0].numel(), self.seg_max, st)
@@ -754,10 +763,48 @@ class HydroSystem:
 
     def pc(self, x: torch.Tensor, y: torch.Tensor, precision: str = "fp64") -> torch.Tensor:
         """y = P^-1 x (tstep.py:950-994)."""
+        if self.nS:
+            self.shell.apply(x, y, "fp64" if precision == "fp64" else self.inner_shell_pc)
+        return self._pc_bodies_fibers(x, y, precision)
+
+    def pc_matvec(self, x: torch.Tensor, z: torch.Tensor, w: torch.Tensor, precision: str = "fp64") -> torch.Tensor:
+        """z = P^-1 x and w = A z.  In FP64 the product with the periphery's
+        dense inverse (bound by HBM) runs on a stream of its own beside the
+        fibers' Oseen sum (bound by the FP64 pipe), which does not read it,
+        where the sum takes at least as long; everything has joined the
+        current stream on return."""
+        if precision != "fp64" or not self.product_beside_sum():
+            return self.matvec(self.pc(x, z, precision), w, precision)
+        main = torch.cuda.current_stream(self.device)
+        if self._side is None:
+            # high priority: the product's few CTAs are placed before the sum's
+            # many, and the stream is never the one a graph is captured on
+            # (ordinary streams repeat after 32)
+            self._side = torch.cuda.Stream(self.device, priority=-1)
+        self._side.wait_stream(main)
+        with torch.cuda.stream(self._side):
+            self.shell.apply(x, z, "fp64", beside=True)
+        self._pc_bodies_fibers(x, z, precision)
+        return self.matvec(z, w, precision, join=self._side)
+
+    def product_beside_sum(self) -> bool:
+        """Whether pc_matvec overlaps.  The product on its part of the SMs is
+        slower alone (18000 rows: 500 us instead of 410), so the sum has to
+        cover it: at 460 G pairs/s and 6.3 TB/s it does from 0.6 pairs per
+        entry of the inverse on.  Time steps with the overlap and without: 512
+        fibers and 6000 periphery nodes (0.8 pairs) 10.4 and 12.2 ms, 300 and
+        3000 (0.9) 3.5 and 3.95 ms, 1000 and 2000 (16) 17.2 and 17.4 ms; below,
+        256 and 6000 (0.26) 5.9 to 6.9 and 6.15 ms, 64 and 6000 (0.04) 4.2 and
+        3.8 ms.  Inverses below 3000 rows take 25 us and gain nothing."""
+        m = 3 * self.nS
+        if m < 3000 or not self.nF or self.shell.pc == "block":
+            return False
+        return self.nF * (0.5 * self.nF + self.nB + self.nS) >= 0.6 * m * m
+
+    def _pc_bodies_fibers(self, x: torch.Tensor, y: torch.Tensor, precision: str) -> torch.Tensor:
+        """The bodies' and fibers' parts of y = P^-1 x."""
         st = _lib.stream_handle(self.device)
         nS = self.nS
-        if nS:
-            self.shell.apply(x, y, "fp64" if precision == "fp64" else self.inner_shell_pc)
         if self.nbody:
             tb = self.body_tmp
             tb.copy_(x[3 * nS:self.o_fib])

@@ -76,3 +76,21 @@ def test_blocks(sizes):
     for b, Mb in enumerate(blocks):
         o = int(lu.voff_h[b])
         _close(got[o:o + sizes[b]], Mb, x[o:o + sizes[b]])
+
+
+@pytest.mark.parametrize("rows,cols,pad,shift", [(1, 2, 0, 0), (9, 65, 1, 1), (593, 130, 0, 0), (4740, 64, 2, 0)])
+def test_product_on_a_part_of_the_sms(rows, cols, pad, shift):
+    from fiber3d_b200 import _lib
+    rng = np.random.default_rng(rows)
+    M, x = rng.normal(size=(rows, cols)), rng.normal(size=cols)
+    ld = cols + pad
+    buf = torch.zeros(shift + rows * ld + 2, dtype=torch.float64, device="cuda")
+    Md = buf[shift:shift + rows * ld].view(rows, ld)
+    Md[:, :cols] = torch.tensor(M)
+    xd = torch.tensor(x, device="cuda")
+    y = torch.full((rows + 1,), float("nan"), dtype=torch.float64, device="cuda")
+    _lib.call("f3d_gemv_beside", _lib.ptr(Md), ld, _lib.ptr(xd), _lib.ptr(y), rows, cols,
+              _lib.stream_handle(y.device))
+    got = y.cpu().numpy()
+    _close(got[:rows], M, x)
+    assert np.isnan(got[rows])
