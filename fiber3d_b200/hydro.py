@@ -784,8 +784,12 @@ class HydroSystem:
         self._side.wait_stream(main)
         with torch.cuda.stream(self._side):
             self.shell.apply(x, z, "fp64", beside=True)
-        self._pc_bodies_fibers(x, z, precision)
-        return self.matvec(z, w, precision, join=self._side)
+        try:
+            self._pc_bodies_fibers(x, z, precision)
+            return self.matvec(z, w, precision, join=self._side)
+        except BaseException:
+            main.wait_stream(self._side)  # x and z are the caller's again
+            raise
 
     def product_beside_sum(self) -> bool:
         """Whether pc_matvec overlaps.  The product on its part of the SMs is
