@@ -665,7 +665,8 @@ __device__ __forceinline__ void products(double (&acc)[3][2][4], const double (*
 // running ahead (9.35 and 51.7 ms); and the warps' column groups: w and w + 4,
 // not 2 w and 2 w + 1, so that the outer boxes of a tile, which lack sources
 // most often, and a short tile's columns spread over the SM's four quarters,
-// each with a tensor core of its own (8.95 and 49.4 ms).  (Operands read 16
+// each with a tensor core of its own (8.95 and 49.4 ms; 8.47 and 48.8 with the
+// order of level 2's boxes, see octant_keys_kernel).  (Operands read 16
 // bytes at a time: 11.3 and 63.3 ms.)  The order of every sum is as it was: at
 // order 8 the check-to-equivalent maps turn a rounding there into 1e-8 of the
 // result.

@@ -9,7 +9,7 @@ namespace f3d {
 // the same part of x, through a ring of its own in shared memory (cp.async; a
 // lane reads back only what it copied, so nothing waits for another lane).
 // Bound by HBM, or by L2 where the matrix stays there: what counts is the bytes
-// in flight, which the ring holds without registers, 48 to 72 KB per SM.
+// in flight, which the rings hold without registers (144 KB per SM for one matrix).
 // Loading through registers, four rows of a warp one after the other behind
 // CTA-wide staging of x, drained the loads at each row and chunk: 82 us for
 // 3600 x 3600, 188 us for 9000 x 9000 and 446 us for 18000 x 18000 from HBM,
