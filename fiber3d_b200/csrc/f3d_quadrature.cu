@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(kKnnThreads) quad_knn_kernel(const double *__r
   int(*pj)[kQuadNbr] = reinterpret_cast<int(*)[kQuadNbr]>(cj + 2);                // [2]
   int *hist = reinterpret_cast<int *>(pj + 2);                                    // kKnnBins
   unsigned *keys0 = reinterpret_cast<unsigned *>(hist + kKnnBins);                // [2][tile + 80]
-  __shared__ unsigned s_min[2][kHalf];
+  __shared__ __align__(16) unsigned s_min[2][kHalf];  // read four at a time
   __shared__ unsigned s_tau[2];
   __shared__ int s_part[kKnnThreads / 32];
   __shared__ int s_bin, s_below, s_ncand[2];
