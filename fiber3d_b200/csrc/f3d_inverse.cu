@@ -240,17 +240,17 @@ __global__ void __launch_bounds__(InvShape<NMAX>::kThreads, 1)
 //    in registers a step is bound by the shared-memory pipe: each warp's best
 //    row is posted and the pivot row read back 16 bytes at a time, about five
 //    cycles an access and warp.)  Partial pivoting: the pivot of step k is the
-//    first row whose |a_ik|, cut to its leading 12 mantissa bits, is largest
-//    among the rows not yet pivoted (a pivot within 2^-12 of the column
-//    maximum).  The key (those bits, then 128 - row) makes the search one
-//    warp max-reduction and a max over the warps; each warp's winner posts
-//    its row, key and reciprocal, so a step needs one barrier (posts double
+//    first row whose |a_ik|, cut to its leading 16 mantissa bits, is largest
+//    among the rows not yet pivoted (a pivot within 2^-16 of the column
+//    maximum).  The key (exponent, those bits, the lane: 32 bits) makes the
+//    search one warp max-reduction and a max over the warps; each warp's winner
+//    posts its row, key and reciprocal, so a step needs one barrier (posts double
 //    buffered by step parity).  Rows are never exchanged: the pivot rows are
 //    recorded instead (perm).
 //  * Update: every other column moves by W R (W the panel after its sweeps,
 //    R the old entries of the panel's 16 pivot rows), the pivot rows
 //    themselves starting from zero: one m16n8k16 step on the FP64 tensor
-//    cores per 16 x 8 tile.  At 128 rows (172 KB: one block per SM) the next
+//    cores per 16 x 8 tile.  At 128 rows (189 KB: one block per SM) the next
 //    panel's columns come first, by all warps, then the rest by half of them
 //    while the others sweep that panel; up to 96 rows two blocks share an SM
 //    and up to 64 rows four, which overlap by themselves.
@@ -285,8 +285,8 @@ __global__ void __launch_bounds__(256, NMAX == 64 ? 4 : (NMAX == 96 ? 2 : 1))
   double *W2 = X + NMAX * S;                         // [kW][NMAX][kWS], by panel parity
   double *Rs = W2 + T::kW * NMAX * T::kWS;           // [16][S]
   __shared__ __align__(16) unsigned s_key[2][4];
-  __shared__ __align__(16) double s_cand[2][NMAX / 32][6];  // each warp's best row of the sub-panel and its
-                                                            // pivot's reciprocal, by step parity
+  __shared__ __align__(16) double s_cand[2][NMAX / 32][6];  // each warp's best row of the sub-panel, its pivot's
+                                                            // reciprocal and its number, by step parity
   __shared__ int s_zero;
   __shared__ int s_perm[NMAX];   // pivot row of step k
   __shared__ int s_step[NMAX];   // step whose pivot is row r (-16: not yet)
@@ -340,29 +340,29 @@ __global__ void __launch_bounds__(256, NMAX == 64 ? 4 : (NMAX == 96 ? 2 : 1))
 #pragma unroll
       for (int jj = 0; jj < 4; ++jj) {
         const int par = jj & 1, k = c0 + s0 + jj;
-        // pivot key: the leading word of |a_ik|, its last 8 bits replaced by
-        // 128 - row (first row among equals; never 0 for a row not yet
-        // pivoted); pivoted rows 0
-        const unsigned key = done ? 0u
-                                  : ((static_cast<unsigned>(__double2hiint(v[jj])) & 0x7fffff00u) |
-                                     static_cast<unsigned>(128 - i));
+        // pivot key: 16 mantissa bits of |a_ik| under its exponent, then the lane
+        // (the first row among equals); never below 32 for a row not yet
+        // pivoted (the cap keeps a NaN from carrying over), pivoted rows 0
+        const unsigned mag = min(static_cast<unsigned>(__double2hiint(v[jj])) << 1, 0xffffffbfu) & ~31u;
+        const unsigned key = done ? 0u : mag + static_cast<unsigned>(63 - lane);
         const double rcp = reciprocal(v[jj]);  // beside the search
         const unsigned wmax = __reduce_max_sync(0xffffffffu, key);
         if (key == wmax) {  // this warp's winner posts its row (live keys are distinct; a warp
-                            // with no live row posts garbage under key 0, which never wins)
-          s_key[par][warp] = wmax;
+                            // with no live row posts garbage under a key that never wins)
+          s_key[par][warp] = (wmax & ~31u) | static_cast<unsigned>(31 - warp);  // the first warp among equals
           double *const c = s_cand[par][warp];
           *reinterpret_cast<double2 *>(c) = make_double2(v[0], v[1]);
           *reinterpret_cast<double2 *>(c + 2) = make_double2(v[2], v[3]);
-          c[4] = rcp;
+          *reinterpret_cast<double2 *>(c + 4) = make_double2(rcp, __hiloint2double(0, i));
         }
         bar();
         const uint4 h = *reinterpret_cast<const uint4 *>(s_key[par]);
         const unsigned best = max(max(h.x, h.y), max(h.z, h.w));
-        const int pr = 128 - static_cast<int>(best & 255u);
+        const double *prow = s_cand[par][31 - static_cast<int>(best & 31u)];
+        const double2 post = *reinterpret_cast<const double2 *>(prow + 4);
+        const double inv = post.x;
+        const int pr = __double2loint(post.y);
         piv[jj] = pr;
-        const double *prow = s_cand[par][pr >> 5];
-        const double inv = prow[4];
         if (i == pr) {
           s_perm[k] = i;
           s_step[i] = k;
