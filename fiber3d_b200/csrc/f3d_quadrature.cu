@@ -606,7 +606,8 @@ __device__ __forceinline__ void tri_pivot(double (&v)[16], TriShared &S, int k, 
   const unsigned mag = static_cast<unsigned>(__double2hiint(v[jj])) & 0x7fffffffu;
   const bool nan = v[jj] != v[jj];
   const unsigned hi = done ? 0u : (nan ? 1u : mag + 2u), lo = nan ? 0u : __double2loint(v[jj]);
-  const double rcp = 1.0 / v[jj];  // beside the search
+  // beside the search; of zero or not a number, the error below, as of 1
+  const double rcp = fabs(v[jj]) > 0.0 ? 1.0 / v[jj] : 1.0;
   const unsigned hmax = __reduce_max_sync(0xffffffffu, hi);
   bool best = hi == hmax;
   const unsigned all = __ballot_sync(0xffffffffu, best);
@@ -644,7 +645,7 @@ __device__ __forceinline__ void tri_pivot(double (&v)[16], TriShared &S, int k, 
   if (pos == pp) {  // the pivot row
     pos = k;
     done = true;
-    if (!(fabs(d) > 0.0)) {  // zero or not a number: an error; go on as if the pivot were 1
+    if (!(fabs(d) > 0.0)) {  // zero or not a number: an error; go on as if the pivot were 1 (rd is)
       record_error(err, F3D_ERR_SINGULAR);
       v[jj] = 1.0;
     }
