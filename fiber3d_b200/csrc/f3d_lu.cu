@@ -27,7 +27,8 @@
 // The trailing matrix stays in global memory; it is L2-resident while the CTA
 // works on it.
 // Solve: one CTA per system (persistent over systems), right-hand side in
-// shared memory, substitution by blocks of 32 unknowns.
+// shared memory, substitution by blocks of 32 unknowns; batches of many small
+// systems by one warp per system.
 #include <algorithm>
 #include <climits>
 
@@ -677,7 +678,7 @@ __global__ void __launch_bounds__(kSvThreads) batched_lu_solve_kernel(const LuSo
       if (warp == 0) {
         double v = lane < kw ? y[k0 + lane] : 0.0;
 #pragma unroll 8
-        for (int j = 0; j < kSvB; ++j) {
+        for (int j = 0; j < kw; ++j) {
           const double xj = __shfl_sync(0xffffffffu, v, j);
           if (lane > j) v = fma(-T[lane * kSvTS + j], xj, v);
         }
@@ -701,7 +702,7 @@ __global__ void __launch_bounds__(kSvThreads) batched_lu_solve_kernel(const LuSo
         const bool plain = fabs(dg) >= 1e-290 && fabs(dg) <= 1e290;
         const double rd = 1.0 / dg;
 #pragma unroll 4
-        for (int j = kSvB - 1; j >= 0; --j) {
+        for (int j = kw - 1; j >= 0; --j) {
           const double q = v * rd;
           double xj = fma(fma(-q, dg, v), rd, q);
           if (!(plain && fabs(q) <= 1e290)) xj = v / dg;
@@ -729,6 +730,83 @@ __global__ void __launch_bounds__(kSvThreads) batched_lu_solve_kernel(const LuSo
       a.queue[1] = 0u;
     }
   }
+}
+
+// A warp per system, a dot product and five shuffles per unknown: slower than
+// the blocks above for one system (92 against 40 us at 64 rows), but an SM holds
+// 48 or 64 systems instead of 16 CTAs whose other warps wait for the one with the
+// triangle, and a small system has no 32 unknowns to fill a block with (see
+// solve_by_warps).
+constexpr int kSolveWarps = 8;
+
+__global__ void __launch_bounds__(kSolveWarps * 32) batched_lu_solve_warp_kernel(const LuSolveArgs a) {
+  extern __shared__ __align__(16) double sv_smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double *y = sv_smem + static_cast<size_t>(warp) * a.max_n;
+  while (true) {
+    int item = 0;
+    if (lane == 0) item = static_cast<int>(atomicAdd(&a.queue[0], 1u));
+    item = __shfl_sync(0xffffffffu, item, 0);
+    if (item >= a.count) break;
+    const int b = a.order ? a.order[item] : item;
+    const int n = a.sizes[b];
+    const double *L = a.LU + a.moff[b];
+    const int32_t *pv = a.piv + a.voff[b];
+    double *x = a.x + a.voff[b];
+    for (int i = lane; i < n; i += 32) y[i] = x[i];
+    __syncwarp();
+    if (lane == 0) {
+      for (int i = 0; i < n; ++i) {
+        const int p = pv[i];
+        if (p != i) { const double t = y[i]; y[i] = y[p]; y[p] = t; }
+      }
+    }
+    __syncwarp();
+    for (int i = 1; i < n; ++i) {  // forward, unit lower
+      const double *row = L + static_cast<int64_t>(i) * n;
+      double s = 0.0;
+      for (int j = lane; j < i; j += 32) s = fma(row[j], y[j], s);
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+      if (lane == 0) y[i] -= s;
+      __syncwarp();
+    }
+    for (int i = n - 1; i >= 0; --i) {  // backward, upper with diagonal
+      const double *row = L + static_cast<int64_t>(i) * n;
+      double s = 0.0;
+      for (int j = i + 1 + lane; j < n; j += 32) s = fma(row[j], y[j], s);
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+      if (lane == 0) y[i] = (y[i] - s) / row[i];
+      __syncwarp();
+    }
+    for (int i = lane; i < n; i += 32) x[i] = y[i];
+    __syncwarp();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(&a.queue[1], 1u) == gridDim.x - 1) {
+      a.queue[0] = 0u;
+      a.queue[1] = 0u;
+    }
+  }
+}
+
+// Whether a batch takes a warp per system: where its systems fill enough of the
+// warps resident at once (`resident`).  A batch costs the CTAs about 0.5 ns a row
+// and system, the warps 1.9 to 2.7 us a row and wave; of blocks with fewer than 32
+// rows, or with few in their last 32, the CTAs gain less.  CTAs and warps, us:
+// 16 rows, 1000 systems 22 and 25, 2000 31 and 27, 50000 580 and 207; 40 rows,
+// 2000 49 and 55, 3000 74 and 61, 10000 221 and 147; 32 rows, 3000 45 and 49, 5000
+// 66 and 59; 64 rows, 5000 147 and 147, 8000 (two waves) 227 and 265, 12000 336 and
+// 285; 128 rows, 2000 141 and 307, 5000 317 and 340, 8000 500 and 635, 12000 741 and
+// 670.  Larger blocks stay with the CTAs (256 rows, 3000: 547 and 777).
+static bool solve_by_warps(int count, int max_n, int resident) {
+  if (max_n > 160 || resident < 1) return false;
+  const int64_t waves = (static_cast<int64_t>(count) + resident - 1) / resident;
+  const int64_t enough = max_n < 32 ? 1500 : max_n == 32 ? 4000 : max_n < 64 ? 2500 : 5000;
+  return count > enough * waves;
 }
 
 static int pick_nb(int max_n) {
@@ -842,8 +920,25 @@ int f3d_batched_lu_solve(const double *LU, const int64_t *matrix_offsets,
   if (count == 0) return F3D_OK;
   if (!LU || !matrix_offsets || !vector_offsets || !sizes || !piv || !x) return F3D_ERR_NULL;
   if (!workspace || workspace_bytes < 256) return F3D_ERR_WORKSPACE;
-  // the limit of the blocks this call takes (one warp's right-hand side of eight)
-  if (8 * static_cast<size_t>(max_n) * sizeof(double) > 200 * 1024) return F3D_ERR_TOO_LARGE;
+  // the limit of the blocks this call takes
+  const size_t warp_smem = f3d::kSolveWarps * static_cast<size_t>(max_n) * sizeof(double);
+  if (warp_smem > 200 * 1024) return F3D_ERR_TOO_LARGE;
+  // queue counters live after the factor's two words
+  f3d::LuSolveArgs a{LU, matrix_offsets, vector_offsets, sizes, order, piv, x,
+                     static_cast<unsigned *>(workspace) + 2, count, max_n};
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (count > 1500 && max_n <= 160) {
+    auto k = f3d::batched_lu_solve_warp_kernel;
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, f3d::kSolveWarps * 32, warp_smem) != cudaSuccess)
+      return F3D_ERR_CUDA;
+    const int ctas = per_sm * f3d::sm_count();
+    if (f3d::solve_by_warps(count, max_n, f3d::kSolveWarps * ctas)) {
+      const int grid = std::min((count + f3d::kSolveWarps - 1) / f3d::kSolveWarps, ctas);
+      k<<<grid, f3d::kSolveWarps * 32, warp_smem, st>>>(a);
+      return f3d::launch_status();
+    }
+  }
   const size_t smem = (static_cast<size_t>((max_n + 1) / 2 * 2) + f3d::kSvB * f3d::kSvTS + 1) * sizeof(double) +
                       static_cast<size_t>(max_n) * sizeof(int32_t);
   auto k = f3d::batched_lu_solve_kernel;
@@ -853,10 +948,7 @@ int f3d_batched_lu_solve(const double *LU, const int64_t *matrix_offsets,
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, f3d::kSvThreads, smem) != cudaSuccess || per_sm < 1)
     per_sm = 1;
   const int grid = std::max(1, std::min(count, per_sm * f3d::sm_count()));
-  // queue counters live after the factor's two words
-  f3d::LuSolveArgs a{LU, matrix_offsets, vector_offsets, sizes, order, piv, x,
-                     static_cast<unsigned *>(workspace) + 2, count, max_n};
-  k<<<grid, f3d::kSvThreads, smem, static_cast<cudaStream_t>(stream)>>>(a);
+  k<<<grid, f3d::kSvThreads, smem, st>>>(a);
   return f3d::launch_status();
 }
 
