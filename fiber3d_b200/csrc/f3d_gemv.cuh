@@ -14,8 +14,8 @@ namespace f3d {
 // CTA-wide staging of x, drained the loads at each row and chunk: 82 us for
 // 3600 x 3600, 188 us for 9000 x 9000 and 446 us for 18000 x 18000 from HBM,
 // against 29, 121 and 410 us (6.3 TB/s) here; four matrices of 1206 in one launch
-// 33 and 12 us; 512 blocks of 128 x 128 29 and 15 us.  (Four rows: the same; eight:
-// 5 % slower at 12000; a quarter of the bytes in flight: 20 %.)
+// 33 and 12 us.  (Four rows: the same; eight: 5 % slower at 12000; a quarter of the
+// bytes in flight: 20 %.)
 constexpr int kGemvRows = 2, kGemvDepth = 6;
 template <int ROWS = kGemvRows, int DEPTH = kGemvDepth>
 constexpr int gemv_ring_doubles() {

@@ -33,7 +33,6 @@
 #include <climits>
 
 #include "f3d_common.cuh"
-#include "f3d_gemv.cuh"
 
 namespace f3d {
 
@@ -489,30 +488,91 @@ __global__ void __launch_bounds__(256, NMAX == 64 ? 4 : (NMAX == 96 ? 2 : 1))
 }
 
 // y_b = M_b x_b for every block b (M row-major n_b x n_b at moff[b], x and y
-// at voff[b]), a CTA per block.  FP64: the block's rows shared out to the warps,
-// which stream them (16-byte copies where the block allows it).
-constexpr int kBlockGemvWarps = 4;
-__global__ void __launch_bounds__(32 * kBlockGemvWarps) block_gemv_kernel(const double *__restrict__ M,
-                                                                          const int64_t *__restrict__ moff,
-                                                                          const int64_t *__restrict__ voff,
-                                                                          const int32_t *__restrict__ sizes, int count,
-                                                                          const double *__restrict__ x,
-                                                                          double *__restrict__ y) {
-  extern __shared__ __align__(16) double gemv_ring[];
-  const int b = blockIdx.x, warp = threadIdx.x >> 5;
+// at voff[b]), a CTA per block, 8 lanes per row, FP64 accumulation.  FP64: ROWS
+// rows 16 apart and U loads a row (16 bytes each where the block is aligned) in
+// flight per lane.  Bound by HBM, or by L2 where the blocks stay there, so what
+// counts is the bytes in flight and, in L2, the instructions beside them; the
+// registers hold both down for small blocks.  1 x 4 up to 16 rows (ROWS x U), 2 x
+// 2 up to 32, 4 x 2 up to 96, 4 x 4 above.  From L2 / from HBM, us, against one
+// load at a time and against rows streamed through cp.async rings: 600 blocks of
+// 128 rows 12 / 25 (27 / 43, 22 / 27), 2000 of 128 47 / 57 (74 / 86, 50 / 61), 600
+// of 96 10 / 18 (12 / 24, 17 / 20), 2000 of 64 12 / 20 (13 / 25, 21 / 25), 10000 of
+// 32 18 / 27 (20 / 31, 42 / 47), 50000 of 8 33 / 47 (35 / 55, 72 / 96), one of 1000
+// 127 / 250 (521 / 1540, 253 / 283).
+template <int ROWS, int U>
+__global__ void __launch_bounds__(128) block_gemv_kernel(const double *__restrict__ M,
+                                                         const int64_t *__restrict__ moff,
+                                                         const int64_t *__restrict__ voff,
+                                                         const int32_t *__restrict__ sizes, int count,
+                                                         const double *__restrict__ x, double *__restrict__ y) {
+  extern __shared__ __align__(16) double xs[];
+  const int b = blockIdx.x;
   if (b >= count) return;
   const int n = sizes[b];
   const double *Mb = M + moff[b], *xb = x + voff[b];
-  double *yb = y + voff[b], *ring = gemv_ring + warp * gemv_ring_doubles();
-  const int lo = warp * n / kBlockGemvWarps, hi = (warp + 1) * n / kBlockGemvWarps;
-  if ((reinterpret_cast<uintptr_t>(Mb) & 15) == 0 && n % 2 == 0)
-    gemv_stream_rows<2>(Mb, xb, yb, lo, hi, n, n, ring);
-  else
-    gemv_stream_rows<1>(Mb, xb, yb, lo, hi, n, n, ring);
+  double *yb = y + voff[b];
+  for (int i = threadIdx.x; i < n; i += blockDim.x) xs[i] = xb[i];
+  __syncthreads();
+  const bool vec = ((reinterpret_cast<uintptr_t>(Mb) & 15) == 0) && (n % 2 == 0);
+  const int sub = threadIdx.x & 7, grp = threadIdx.x >> 3;  // lane within the row group, 16 row groups
+  for (int r0 = 0; r0 < n; r0 += 16 * ROWS) {
+    const int r = r0 + grp;
+    double s[ROWS];
+#pragma unroll
+    for (int q = 0; q < ROWS; ++q) s[q] = 0.0;
+    if (vec) {
+      for (int c0 = 2 * sub; c0 < n; c0 += 16 * U) {
+        double2 v[ROWS][U];
+#pragma unroll
+        for (int q = 0; q < ROWS; ++q)
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int c = c0 + 16 * u;
+            v[q][u] = make_double2(0.0, 0.0);
+            if (c < n && r + 16 * q < n)
+              v[q][u] = *reinterpret_cast<const double2 *>(Mb + static_cast<int64_t>(r + 16 * q) * n + c);
+          }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int c = c0 + 16 * u;
+          if (c < n) {
+            const double2 w = *reinterpret_cast<const double2 *>(xs + c);
+#pragma unroll
+            for (int q = 0; q < ROWS; ++q) s[q] = fma(v[q][u].y, w.y, fma(v[q][u].x, w.x, s[q]));
+          }
+        }
+      }
+    } else {
+      for (int c0 = sub; c0 < n; c0 += 8 * U) {
+        double v[ROWS][U];
+#pragma unroll
+        for (int q = 0; q < ROWS; ++q)
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int c = c0 + 8 * u;
+            v[q][u] = c < n && r + 16 * q < n ? Mb[static_cast<int64_t>(r + 16 * q) * n + c] : 0.0;
+          }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int c = c0 + 8 * u;
+          if (c < n) {
+#pragma unroll
+            for (int q = 0; q < ROWS; ++q) s[q] = fma(v[q][u], xs[c], s[q]);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < ROWS; ++q) {
+#pragma unroll
+      for (int off = 1; off < 8; off <<= 1) s[q] += __shfl_xor_sync(0xffffffffu, s[q], off);
+      if (sub == 0 && r + 16 * q < n) yb[r + 16 * q] = s[q];
+    }
+  }
 }
 
-// The FP32 copy: 8 lanes per row (16-byte loads where the block is aligned),
-// FP64 accumulation.
+// The FP32 copy: one row and one load (16 bytes where the block is aligned) at a
+// time per lane, FP64 accumulation.
 __global__ void __launch_bounds__(128) block_gemv_f32_kernel(const float *__restrict__ M,
                                                              const int64_t *__restrict__ moff,
                                                              const int64_t *__restrict__ voff,
@@ -615,7 +675,11 @@ int f3d_block_gemv(int precision, const void *M, const int64_t *matrix_offsets,
   if (smem > 48 * 1024) return F3D_ERR_TOO_LARGE;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (precision == F3D_FP64) {
-    f3d::block_gemv_kernel<<<count, 32 * f3d::kBlockGemvWarps, f3d::kBlockGemvWarps * f3d::kGemvWarpSmem, st>>>(
+    auto kernel = max_n <= 16 ? f3d::block_gemv_kernel<1, 4>
+                  : max_n <= 32 ? f3d::block_gemv_kernel<2, 2>
+                  : max_n <= 96 ? f3d::block_gemv_kernel<4, 2>
+                                : f3d::block_gemv_kernel<4, 4>;
+    kernel<<<count, 128, smem, st>>>(
         static_cast<const double *>(M), matrix_offsets, vector_offsets, sizes, count, x, y);
   } else if (precision == F3D_FP32C) {
     f3d::block_gemv_f32_kernel<<<count, 128, smem, st>>>(
