@@ -241,8 +241,9 @@ __global__ void __launch_bounds__(32 * kGemvWarps) gemv_kernel(const double *__r
 }
 
 // count square FP64 matrices in one launch: matrix b (n[b] x n[b], row-major
-// at M + m_off[b]) times x + x_off[b] into y + y_off[b]; blockIdx.y = b.
-template <int VEC>
+// at M + m_off[b]) times x + x_off[b] into y + y_off[b]; blockIdx.y = b.  The rows
+// go to the warps in groups of ROWS, so that no group is cut.
+template <int VEC, int ROWS, int DEPTH>
 __global__ void __launch_bounds__(32 * kGemvWarps) gemv_batched_kernel(const double *__restrict__ M,
                                                                        const int64_t *__restrict__ m_off,
                                                                        const int64_t *__restrict__ n,
@@ -251,11 +252,12 @@ __global__ void __launch_bounds__(32 * kGemvWarps) gemv_batched_kernel(const dou
                                                                        const double *__restrict__ x, double *y) {
   extern __shared__ __align__(16) double gemv_ring[];
   const int b = blockIdx.y, warp = threadIdx.x >> 5;
-  const int64_t nb = n[b];
+  const int64_t nb = n[b], groups = (nb + ROWS - 1) / ROWS;
   const int64_t w = static_cast<int64_t>(blockIdx.x) * kGemvWarps + warp;
   const int64_t nw = static_cast<int64_t>(gridDim.x) * kGemvWarps;
-  gemv_stream_rows<VEC>(M + m_off[b], x + x_off[b], y + y_off[b], w * nb / nw, (w + 1) * nb / nw, nb, nb,
-                        gemv_ring + warp * gemv_ring_doubles());
+  gemv_stream_rows<VEC, ROWS, DEPTH>(M + m_off[b], x + x_off[b], y + y_off[b], ROWS * (w * groups / nw),
+                                     min(nb, ROWS * ((w + 1) * groups / nw)), nb, nb,
+                                     gemv_ring + warp * gemv_ring_doubles<ROWS, DEPTH>());
 }
 
 constexpr size_t kGemvSmem = kGemvWarps * kGemvWarpSmem;
@@ -602,14 +604,29 @@ int f3d_gemv_batched(const double *M, const int64_t *m_off, const int64_t *n, co
   if (!M || !m_off || !n || !x_off || !y_off || !x || !y) return F3D_ERR_NULL;
   if (vec && reinterpret_cast<uintptr_t>(M) % 16 != 0) return F3D_ERR_ALIGN;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // two CTAs per SM in all, at least a row for each warp
+  // three CTAs per SM in all, at least a row for each warp
+  const int64_t ctas = 3 * static_cast<int64_t>(f3d::sm_count());
   const int64_t per = std::max<int64_t>(1, std::min<int64_t>((max_n + f3d::kGemvWarps - 1) / f3d::kGemvWarps,
-                                                             (static_cast<int64_t>(f3d::sm_count()) * 2 + count - 1) / count));
+                                                             (ctas + count - 1) / count));
   const dim3 grid(static_cast<unsigned>(per), static_cast<unsigned>(count));
-  auto kernel = vec ? f3d::gemv_batched_kernel<2> : f3d::gemv_batched_kernel<1>;
-  if (!f3d::gemv_allow(kernel)) return F3D_ERR_CUDA;
-  kernel<<<grid, 32 * f3d::kGemvWarps, f3d::kGemvSmem, st>>>(M, m_off, n, x_off, y_off, x, y);
-  return f3d::launch_status();
+  auto launch = [&](auto kernel, size_t warp_ring) {
+    const size_t smem = f3d::kGemvWarps * warp_ring * sizeof(double);
+    if (!f3d::gemv_allow(kernel, smem)) return static_cast<int>(F3D_ERR_CUDA);
+    kernel<<<grid, 32 * f3d::kGemvWarps, smem, st>>>(M, m_off, n, x_off, y_off, x, y);
+    return f3d::launch_status();
+  };
+  // Groups of four rows share one copy of x and of a warp's other work; with
+  // fewer than three rows a warp they leave warps idle, and rows two at a time
+  // are faster.  From L2 / from HBM, us, fours and twos: 40 matrices of 306 rows 12
+  // / 14 and 12 / 16, 20 of 606 14 / 23 and 18 / 23, 12 of 1206 33 / 43 and 33 /
+  // 41, 100 of 906 111 / 125 and 125 / 137; 4 of 1206 15 / 23 and 15 / 18, 4 of 606
+  // 11 / 14 and 9 / 10.  (Twos with two CTAs per SM and uncut shares of rows, as
+  // before: 14 / 16, 21 / 25, 39 / 47, 150 / 165; 15 / 21, 9 / 10.)
+  if (static_cast<int64_t>(count) * max_n >= 3 * f3d::kGemvWarps * ctas)
+    return vec ? launch(f3d::gemv_batched_kernel<2, 4, 4>, f3d::gemv_ring_doubles<4, 4>())
+               : launch(f3d::gemv_batched_kernel<1, 4, 4>, f3d::gemv_ring_doubles<4, 4>());
+  return vec ? launch(f3d::gemv_batched_kernel<2, f3d::kGemvRows, f3d::kGemvDepth>, f3d::gemv_ring_doubles())
+             : launch(f3d::gemv_batched_kernel<1, f3d::kGemvRows, f3d::kGemvDepth>, f3d::gemv_ring_doubles());
 }
 
 int f3d_gemv_beside(const double *M, int64_t ld, const double *x, double *y, int64_t rows, int64_t cols,
