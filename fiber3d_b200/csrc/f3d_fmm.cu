@@ -38,6 +38,7 @@
 //     non-empty leaf on average (2 <= depth <= 8).
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <vector>
 
 #include "f3d_common.cuh"
@@ -237,7 +238,7 @@ static int scan_exclusive(int *a, int64_t n, int *tile_sums, int *d_total, cudaS
   const int ntiles = static_cast<int>((n + kScanTile - 1) / kScanTile);
   scan_tiles_kernel<<<ntiles, 1024, 0, st>>>(a, n, tile_sums);
   scan_sums_kernel<<<1, 1024, 0, st>>>(tile_sums, ntiles, d_total);
-  scan_add_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(a, n, tile_sums);
+  if (ntiles > 1) scan_add_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(a, n, tile_sums);
   return launch_status();
 }
 
@@ -909,10 +910,11 @@ __global__ void near_count_kernel(const int64_t *__restrict__ start, const int64
 }
 
 // leaf of each item from the items' offsets
-__global__ void near_items_kernel(const int *__restrict__ off, int nleaf, int nitems, int *leaf) {
+__global__ void near_items_kernel(const int64_t *__restrict__ start, const int64_t *__restrict__ end,
+                                  const int *__restrict__ off, int nleaf, int *leaf) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nleaf) return;
-  const int e = i + 1 < nleaf ? off[i + 1] : nitems;
+  const int e = off[i] + static_cast<int>((end[i] - start[i] + kNearTargets - 1) / kNearTargets);
   for (int k = off[i]; k < e; ++k) leaf[k] = i;
 }
 
@@ -1232,6 +1234,7 @@ int finish_table(f3d_fmm *h, int64_t nkeys, DevBuf &table, DevBuf &keys, int *co
 
 int build_tree(f3d_fmm *h, cudaStream_t st) {
   int rc;
+  h->nitems = 0;
   // depth: the smallest with at most max_pts sources per non-empty leaf
   if ((rc = reserve(h->scalars, 64 * sizeof(int)))) return rc;
   if (cudaMemsetAsync(h->scalars.p, 0, 64 * sizeof(int), st) != cudaSuccess) return F3D_ERR_CUDA;
@@ -1278,10 +1281,9 @@ int build_tree(f3d_fmm *h, cudaStream_t st) {
   if ((rc = reserve(h->sl_start, rs)) || (rc = reserve(h->sl_end, rs)) || (rc = reserve(h->dl_start, rs)) ||
       (rc = reserve(h->dl_end, rs)) || (rc = reserve(h->trg_start, rt)) || (rc = reserve(h->trg_end, rt)))
     return rc;
+  // (a target leaf has targets, so its range is always written)
   for (DevBuf *b : {&h->sl_start, &h->sl_end, &h->dl_start, &h->dl_end})
     if (cudaMemsetAsync(b->p, 0, rs, st) != cudaSuccess) return F3D_ERR_CUDA;
-  for (DevBuf *b : {&h->trg_start, &h->trg_end})
-    if (cudaMemsetAsync(b->p, 0, rt, st) != cudaSuccess) return F3D_ERR_CUDA;
   if (h->nsl)
     leaf_ranges_kernel<<<blocks(h->nsl), 256, 0, st>>>(as<uint64_t>(h->kv_sl), h->nsl, shift, as<int>(leaf.src_table),
                                                        as<int64_t>(h->sl_start), as<int64_t>(h->sl_end));
@@ -1291,17 +1293,21 @@ int build_tree(f3d_fmm *h, cudaStream_t st) {
   leaf_ranges_kernel<<<blocks(h->ntrg), 256, 0, st>>>(as<uint64_t>(h->kv_trg), h->ntrg, shift, as<int>(leaf.trg_table),
                                                       as<int64_t>(h->trg_start), as<int64_t>(h->trg_end));
   if ((rc = launch_status())) return rc;
-  // near-field items: at most kNearTargets targets of one leaf each
+  // near-field items: at most kNearTargets targets of one leaf each (their number
+  // is read at the end, with the far field's; a leaf has at most one item more
+  // than its share of all targets, which bounds the list)
+  int *const item_total = as<int>(h->scalars) + 50;
   {
-    if ((rc = reserve(h->item_off, static_cast<size_t>(leaf.ntrg) * sizeof(int)))) return rc;
+    const size_t most = static_cast<size_t>(h->ntrg / kNearTargets + leaf.ntrg);
+    if ((rc = reserve(h->item_off, static_cast<size_t>(leaf.ntrg) * sizeof(int))) ||
+        (rc = reserve(h->item_leaf, most * sizeof(int))))
+      return rc;
     near_count_kernel<<<blocks(leaf.ntrg), 256, 0, st>>>(as<int64_t>(h->trg_start), as<int64_t>(h->trg_end), leaf.ntrg,
                                                          as<int>(h->item_off));
     if ((rc = launch_status())) return rc;
-    if ((rc = scan_exclusive(as<int>(h->item_off), leaf.ntrg, as<int>(h->tile_sums), as<int>(h->scalars), st))) return rc;
-    if ((rc = sync_read(&h->nitems, h->scalars.p, sizeof(int), st))) return rc;
-    if ((rc = reserve(h->item_leaf, static_cast<size_t>(h->nitems) * sizeof(int)))) return rc;
-    near_items_kernel<<<blocks(leaf.ntrg), 256, 0, st>>>(as<int>(h->item_off), leaf.ntrg, h->nitems,
-                                                         as<int>(h->item_leaf));
+    if ((rc = scan_exclusive(as<int>(h->item_off), leaf.ntrg, as<int>(h->tile_sums), item_total, st))) return rc;
+    near_items_kernel<<<blocks(leaf.ntrg), 256, 0, st>>>(as<int64_t>(h->trg_start), as<int64_t>(h->trg_end),
+                                                         as<int>(h->item_off), leaf.ntrg, as<int>(h->item_leaf));
     if ((rc = launch_status())) return rc;
   }
   // upper levels: parents of the boxes below
@@ -1352,9 +1358,14 @@ int build_tree(f3d_fmm *h, cudaStream_t st) {
       count_m2l_kernel<<<blocks(lv.ntrg), 256, 0, st>>>(as<int>(lv.trg_keys), lv.ntrg, as<int>(lv.src_table), l, pc);
   }
   if ((rc = launch_status())) return rc;
-  unsigned long long pairs = 0;
-  if ((rc = sync_read(&pairs, pc, sizeof(pairs), st))) return rc;
-  h->m2l_pairs = static_cast<int64_t>(pairs);
+  struct {
+    unsigned long long pairs;
+    int items;
+  } totals{};
+  static_assert(offsetof(decltype(totals), items) == 2 * sizeof(int), "scalars 48 to 50");
+  if ((rc = sync_read(&totals, pc, offsetof(decltype(totals), items) + sizeof(int), st))) return rc;
+  h->m2l_pairs = static_cast<int64_t>(totals.pairs);
+  h->nitems = totals.items;
   return F3D_OK;
 }
 
