@@ -319,7 +319,7 @@ def solve_system(system, tol=1e-8, restart=100, maxiter=200, x0=None, mixed=Fals
         x, info, its, hist = g.solve(lambda a, o: system.matvec(a, o, "fp64"),
                                      lambda a, o: system.pc(a, o, "fp64"), b, x0=x0, rtol=tol,
                                      maxiter=maxiter, use_graph=use_graph, key="fp64", r0=r0,
-                                     pc_matvec=getattr(system, "pc_matvec", None))
+                                     pc_matvec=system.pc_matvec if hasattr(type(system), "pc_matvec") else None)
         return {"x": x, "info": info, "iterations": its, "history": hist, "refinements": 0,
                 "seconds": time.perf_counter() - t0}
     # mixed: FP32C inner solves; outer residuals FP32C while the bound holds

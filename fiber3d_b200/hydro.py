@@ -329,6 +329,11 @@ class _PairCall:
                   _lib.stream_handle(a["out"].device))
 
 
+def _own(obj, cls, *names) -> bool:
+    """Whether obj's methods of these names are cls's own."""
+    return all(getattr(type(obj), k, None) is getattr(cls, k) and k not in vars(obj) for k in names)
+
+
 class HydroSystem:
     """Device linear system of one time step: ``rhs``, :meth:`matvec`,
     :meth:`pc` (the right preconditioner P^-1) and :meth:`solve`."""
@@ -772,9 +777,12 @@ class HydroSystem:
         dense inverse (bound by HBM) runs on a stream of its own beside the
         fibers' Oseen sum (bound by the FP64 pipe), which does not read it,
         where the sum takes at least as long; everything has joined the
-        current stream on return."""
-        if precision != "fp64" or not self.product_beside_sum():
-            return self.matvec(self.pc(x, z, precision), w, precision)
+        current stream on return.  A pc, matvec or shell.apply of a subclass or
+        of the instance is called as it is, one after the other."""
+        if (precision != "fp64" or not self.product_beside_sum() or not _own(self, HydroSystem, "pc", "matvec")
+                or not _own(self.shell, ShellOperator, "apply")):
+            self.pc(x, z, precision)
+            return self.matvec(z, w, precision)
         main = torch.cuda.current_stream(self.device)
         if self._side is None:
             # high priority: the product's few CTAs are placed before the sum's
