@@ -238,14 +238,16 @@ __global__ void __launch_bounds__(InvShape<NMAX>::kThreads, 1)
 //    tile.  (The chain of pivots bounds the kernel, and with all 16 columns
 //    in registers a step is bound by the shared-memory pipe: each warp's best
 //    row is posted and the pivot row read back 16 bytes at a time, about five
-//    cycles an access and warp.)  Partial pivoting: the pivot of step k is the
-//    first row whose |a_ik|, cut to its leading 16 mantissa bits, is largest
-//    among the rows not yet pivoted (a pivot within 2^-16 of the column
-//    maximum).  The key (exponent, those bits, the lane: 32 bits) makes the
-//    search one warp max-reduction and a max over the warps; each warp's winner
-//    posts its row, key and reciprocal, so a step needs one barrier (posts double
-//    buffered by step parity).  Rows are never exchanged: the pivot rows are
-//    recorded instead (perm).
+//    cycles an access and warp.)  Partial pivoting: the pivot of step k is a
+//    row whose |a_ik|, cut to its leading 16 mantissa bits, is largest among the
+//    rows not yet pivoted (a pivot within 2^-16 of the column maximum; among
+//    equals the first lane, then the first warp).  The key (exponent, those bits,
+//    the lane: 32 bits) makes the search one warp max-reduction and a max over
+//    the warps; each warp's winner posts its row, key and reciprocal, so a step
+//    needs one barrier (posts double buffered by step parity).  (12 bits: 249
+//    us for 512 blocks of 128; the row posted beside its pivot instead of read
+//    from the key: 265.)  Rows are never exchanged: the pivot rows are recorded
+//    instead (perm).
 //  * Update: every other column moves by W R (W the panel after its sweeps,
 //    R the old entries of the panel's 16 pivot rows), the pivot rows
 //    themselves starting from zero: one m16n8k16 step on the FP64 tensor
@@ -253,9 +255,9 @@ __global__ void __launch_bounds__(InvShape<NMAX>::kThreads, 1)
 //    panel's columns come first, by all warps, then the rest by half of them
 //    while the others sweep that panel; up to 96 rows two blocks share an SM
 //    and up to 64 rows four, which overlap by themselves.
-// 512 blocks: 250 us at 128 rows, 115 at 96, 45 at 64, against 307, 286 (by the
+// 512 blocks: 253 us at 128 rows, 118 at 96, 43 at 64, against 307, 286 (by the
 // 128-row kernel) and 71 us with 16-column sweeps in registers and the update
-// after them; one block of 128: 65 us, 78 before.  (The block in global memory
+// after them; one block of 128: 62 us, 78 before.  (The block in global memory
 // with four CTAs per SM: 266 us.)
 // Sweeping pivot (perm[k], k) for every k leaves X with X[perm[k], j] =
 // (PA)^-1 (k, j), so A^-1 (k, perm[j]) = X[perm[k], j].
@@ -284,8 +286,8 @@ __global__ void __launch_bounds__(256, NMAX == 64 ? 4 : (NMAX == 96 ? 2 : 1))
   double *W2 = X + NMAX * S;                         // [kW][NMAX][kWS], by panel parity
   double *Rs = W2 + T::kW * NMAX * T::kWS;           // [16][S]
   __shared__ __align__(16) unsigned s_key[2][4];
-  __shared__ __align__(16) double s_cand[2][NMAX / 32][6];  // each warp's best row of the sub-panel, its pivot's
-                                                            // reciprocal and its number, by step parity
+  __shared__ __align__(16) double s_cand[2][NMAX / 32][6];  // each warp's best row of the sub-panel and its
+                                                            // pivot's reciprocal, by step parity
   __shared__ int s_zero;
   __shared__ int s_perm[NMAX];   // pivot row of step k
   __shared__ int s_step[NMAX];   // step whose pivot is row r (-16: not yet)
@@ -315,7 +317,8 @@ __global__ void __launch_bounds__(256, NMAX == 64 ? 4 : (NMAX == 96 ? 2 : 1))
   if (tid == 0) s_zero = INT_MAX;
   __syncthreads();
   int first_zero = 0;  // the first zero pivot this thread's row was (a row is a pivot once)
-  bool done = false;   // this thread's row has been a pivot
+  // this thread's row in the pivot search; all 0 once it has been a pivot
+  unsigned key_mask = 0x7ffffff0u, key_add = 63u - lane;
   constexpr int kRT = NMAX / 16, kCT = NMAX / 8, kPW = NMAX / 32;
   const int g = lane >> 2, t = lane & 3;
 
@@ -339,33 +342,32 @@ __global__ void __launch_bounds__(256, NMAX == 64 ? 4 : (NMAX == 96 ? 2 : 1))
 #pragma unroll
       for (int jj = 0; jj < 4; ++jj) {
         const int par = jj & 1, k = c0 + s0 + jj;
-        // pivot key: 16 mantissa bits of |a_ik| under its exponent, then the lane
-        // (the first row among equals); never below 32 for a row not yet
-        // pivoted (the cap keeps a NaN from carrying over), pivoted rows 0
-        const unsigned mag = min(static_cast<unsigned>(__double2hiint(v[jj])) << 1, 0xffffffbfu) & ~31u;
-        const unsigned key = done ? 0u : mag + static_cast<unsigned>(63 - lane);
+        // pivot key: exponent and 16 mantissa bits of |a_ik| (plus one), then the
+        // lane (the first among equals): at least 32 for a row not yet pivoted,
+        // else 0 (a NaN whose bits are all set wraps; see the end)
+        const unsigned key = 2u * (static_cast<unsigned>(__double2hiint(v[jj])) & key_mask) + key_add;
         const double rcp = reciprocal(v[jj]);  // beside the search
         const unsigned wmax = __reduce_max_sync(0xffffffffu, key);
         if (key == wmax) {  // this warp's winner posts its row (live keys are distinct; a warp
-                            // with no live row posts garbage under a key that never wins)
-          s_key[par][warp] = (wmax & ~31u) | static_cast<unsigned>(31 - warp);  // the first warp among equals
+                            // with no live row posts garbage under key 0, which never wins)
+          s_key[par][warp] = wmax;
           double *const c = s_cand[par][warp];
           *reinterpret_cast<double2 *>(c) = make_double2(v[0], v[1]);
           *reinterpret_cast<double2 *>(c + 2) = make_double2(v[2], v[3]);
-          *reinterpret_cast<double2 *>(c + 4) = make_double2(rcp, __hiloint2double(0, i));
+          c[4] = rcp;
         }
         bar();
         const uint4 h = *reinterpret_cast<const uint4 *>(s_key[par]);
         const unsigned best = max(max(h.x, h.y), max(h.z, h.w));
-        const double *prow = s_cand[par][31 - static_cast<int>(best & 31u)];
-        const double2 post = *reinterpret_cast<const double2 *>(prow + 4);
-        const double inv = post.x;
-        const int pr = __double2loint(post.y);
+        const int bw = h.x == best ? 0 : (h.y == best ? 1 : (h.z == best ? 2 : 3));
+        const int pr = 32 * bw + 31 - static_cast<int>(best & 31u);
+        const double *prow = s_cand[par][bw];
+        const double inv = prow[4];
         piv[jj] = pr;
         if (i == pr) {
           s_perm[k] = i;
           s_step[i] = k;
-          done = true;
+          key_mask = key_add = 0u;
           if (first_zero == 0 && !(fabs(v[jj]) >= 2.2250738585072014e-308)) first_zero = k + 1;
 #pragma unroll
           for (int j = 0; j < 4; ++j) v[j] = (j == jj) ? inv : v[j] * inv;
@@ -473,11 +475,12 @@ __global__ void __launch_bounds__(256, NMAX == 64 ? 4 : (NMAX == 96 ? 2 : 1))
     }
   }
   __syncthreads();
-  // A^-1 (k, c) = X[perm[k], step[c]]: coalesced stores of the block's rows
+  // A^-1 (k, c) = X[perm[k], step[c]]: coalesced stores of the block's rows (a row
+  // that a wrapped key kept from being a pivot has no step)
   float *M32 = A32 ? A32 + moff[b] : nullptr;
   for (int e = tid; e < n * n; e += T::kThreads) {
     const int k = e / n, c = e % n;
-    const double v = X[s_perm[k] * S + s_step[c]];
+    const double v = X[s_perm[k] * S + max(s_step[c], 0)];
     M[e] = v;
     if (M32) M32[e] = static_cast<float>(v);
   }
