@@ -797,15 +797,20 @@ __global__ void __launch_bounds__(kSolveWarps * 32) batched_lu_solve_warp_kernel
 // warps resident at once (`resident`).  A batch costs the CTAs about 0.5 ns a row
 // and system, the warps 1.9 to 2.7 us a row and wave; of blocks with fewer than 32
 // rows, or with few in their last 32, the CTAs gain less.  CTAs and warps, us:
-// 16 rows, 1000 systems 22 and 25, 2000 31 and 27, 50000 580 and 207; 40 rows,
-// 2000 49 and 55, 3000 74 and 61, 10000 221 and 147; 32 rows, 3000 45 and 49, 5000
-// 66 and 59; 64 rows, 5000 147 and 147, 8000 (two waves) 227 and 265, 12000 336 and
+// 8 rows, 1000 systems 16 and 16, 1500 20 and 16; 16 rows, 1000 22 and 25, 2000 31
+// and 27, 50000 580 and 207; 40 rows, 2000 49 and 55, 3000 74 and 61, 10000 221 and
+// 147; 32 rows, 3000 45 and 49, 5000 66 and 59; 72 rows, 3000 135 and 154, 5000 193
+// and 172; 64 rows, 5000 147 and 147, 8000 (two waves) 227 and 265, 12000 336 and
 // 285; 128 rows, 2000 141 and 307, 5000 317 and 340, 8000 500 and 635, 12000 741 and
 // 670.  Larger blocks stay with the CTAs (256 rows, 3000: 547 and 777).
 static bool solve_by_warps(int count, int max_n, int resident) {
   if (max_n > 160 || resident < 1) return false;
   const int64_t waves = (static_cast<int64_t>(count) + resident - 1) / resident;
-  const int64_t enough = max_n < 32 ? 1500 : max_n == 32 ? 4000 : max_n < 64 ? 2500 : 5000;
+  const int64_t enough = max_n <= 12                   ? 1000
+                         : max_n < 32                  ? 1500
+                         : max_n < 64 && max_n != 32   ? 2500
+                         : max_n < 96 && max_n != 64   ? 4000
+                                                       : 5000;
   return count > enough * waves;
 }
 
@@ -927,7 +932,7 @@ int f3d_batched_lu_solve(const double *LU, const int64_t *matrix_offsets,
   f3d::LuSolveArgs a{LU, matrix_offsets, vector_offsets, sizes, order, piv, x,
                      static_cast<unsigned *>(workspace) + 2, count, max_n};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (count > 1500 && max_n <= 160) {
+  if (count > 1000 && max_n <= 160) {
     auto k = f3d::batched_lu_solve_warp_kernel;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, f3d::kSolveWarps * 32, warp_smem) != cudaSuccess)
