@@ -246,8 +246,8 @@ __global__ void __launch_bounds__(kLuThreads) batched_lu_factor_kernel(const LuA
 //    the trailing update gathers them by `phys`, 16 x 32 outputs per warp
 //    with one m16n8k16 step per 16 x 8 tile, operands from the panel and U12
 //    in shared memory, the matrix itself from L2.
-// 256 threads, 80 registers and at most 79 KB per CTA leave three blocks per
-// SM, whose pivot chains overlap.  (128 threads with two rows each: 1.95 ms
+// 256 threads, 80 registers and, up to 224 rows, at most 70 KB per CTA leave three
+// blocks per SM, whose pivot chains overlap; above (78 KB with 256 rows) two.  (128 threads with two rows each: 1.95 ms
 // on the blocks below; every thread scanning the warps' keys and forming the
 // pivot's reciprocal after the barrier: 1.54 ms; 64-bit keys posted in three
 // words: 1.37 ms.)  Measured on 2000 blocks of 64-256 rows (7.2 Gflop):

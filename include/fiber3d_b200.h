@@ -613,7 +613,7 @@ int f3d_gemv_batched(const double *M, const int64_t *m_off, const int64_t *n, co
    the explicit inverse of the periphery operator (tstep/tstep.py:957-958). */
 int f3d_gemv(int precision, const void *M, int64_t ld, const double *x, double *y,
              int64_t rows, int64_t cols, void *stream);
-/* The FP64 product on a part of each SM (one CTA of 256 threads and 72 KB), for a
+/* The FP64 product on a part of each SM (one CTA of 128 threads and 54 KB), for a
    stream that runs beside a kernel bound by the FP64 units. */
 int f3d_gemv_beside(const double *M, int64_t ld, const double *x, double *y, int64_t rows,
                     int64_t cols, void *stream);
