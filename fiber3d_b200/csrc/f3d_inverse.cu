@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(256, NMAX == 64 ? 4 : (NMAX == 96 ? 2 : 1))
                                                             // pivot's reciprocal, by step parity
   __shared__ int s_zero;
   __shared__ int s_perm[NMAX];   // pivot row of step k
-  __shared__ int s_step[NMAX];   // step whose pivot is row r (-16: not yet)
+  __shared__ int s_step[NMAX];   // step whose pivot is row r (NMAX: not yet)
   const int b = blockIdx.x;
   if (b >= count) return;
   const int n = sizes[b];
@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(256, NMAX == 64 ? 4 : (NMAX == 96 ? 2 : 1))
       X[r * S + c] = (r < n && c < n) ? from[r * ldm + c] : (r == c ? 1.0 : 0.0);
     }
   }
-  for (int r = tid; r < NMAX; r += T::kThreads) s_step[r] = -16;
+  for (int r = tid; r < NMAX; r += T::kThreads) s_step[r] = NMAX;
   if (tid < 8) s_key[tid >> 2][tid & 3] = 0u;
   if (tid == 0) s_zero = INT_MAX;
   __syncthreads();
@@ -476,11 +476,11 @@ __global__ void __launch_bounds__(256, NMAX == 64 ? 4 : (NMAX == 96 ? 2 : 1))
   }
   __syncthreads();
   // A^-1 (k, c) = X[perm[k], step[c]]: coalesced stores of the block's rows (a row
-  // that a wrapped key kept from being a pivot has no step)
+  // that a wrapped key kept from being a pivot reads its padding, column NMAX)
   float *M32 = A32 ? A32 + moff[b] : nullptr;
   for (int e = tid; e < n * n; e += T::kThreads) {
     const int k = e / n, c = e % n;
-    const double v = X[s_perm[k] * S + max(s_step[c], 0)];
+    const double v = X[s_perm[k] * S + s_step[c]];
     M[e] = v;
     if (M32) M32[e] = static_cast<float>(v);
   }
