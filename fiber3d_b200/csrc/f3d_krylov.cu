@@ -616,13 +616,14 @@ int f3d_gemv_batched(const double *M, const int64_t *m_off, const int64_t *n, co
     return f3d::launch_status();
   };
   // Groups of four rows share one copy of x and of a warp's other work; with
-  // fewer than three rows a warp they leave warps idle, and rows two at a time
+  // hardly more than two rows a warp they leave warps idle, and rows two at a time
   // are faster.  From L2 / from HBM, us, fours and twos: 40 matrices of 306 rows 12
-  // / 14 and 12 / 16, 20 of 606 14 / 23 and 18 / 23, 12 of 1206 33 / 43 and 33 /
-  // 41, 100 of 906 111 / 125 and 125 / 137; 4 of 1206 15 / 23 and 15 / 18, 4 of 606
-  // 11 / 14 and 9 / 10.  (Twos with two CTAs per SM and uncut shares of rows, as
-  // before: 14 / 16, 21 / 25, 39 / 47, 150 / 165; 15 / 21, 9 / 10.)
-  if (static_cast<int64_t>(count) * max_n >= 3 * f3d::kGemvWarps * ctas)
+  // / 15 and 12 / 16, 20 of 606 14 / 23 and 18 / 23, 40 of 906 51 / 64 and 55 / 69,
+  // 9 of 906 (2.3 rows a warp) 16 / 25 and 21 / 25, 8 of 1206 (2.7) 21 / 31 and 25 /
+  // 33; 6 of 1206 (2.04) 18 / 28 and 19 / 25, 4 of 1206 14 / 23 and 14 / 19, 4 of
+  // 606 10 / 14 and 10 / 10.  (Twos with two CTAs per SM and uncut shares of rows,
+  // as before: 14 / 16, 21 / 27, 62 / 77, 21 / 25, 22 / 31; 24 / 30, 16 / 21, 10 / 10.)
+  if (10 * static_cast<int64_t>(count) * max_n >= 21 * f3d::kGemvWarps * ctas)
     return vec ? launch(f3d::gemv_batched_kernel<2, 4, 4>, f3d::gemv_ring_doubles<4, 4>())
                : launch(f3d::gemv_batched_kernel<1, 4, 4>, f3d::gemv_ring_doubles<4, 4>());
   return vec ? launch(f3d::gemv_batched_kernel<2, f3d::kGemvRows, f3d::kGemvDepth>, f3d::gemv_ring_doubles())

@@ -1,5 +1,5 @@
 """Several FP64 products in one launch on both sides of the rule that takes four
-rows at a time (three rows a warp over three CTAs of eight warps per SM), with
+rows at a time (2.1 rows a warp over three CTAs of eight warps per SM), with
 sizes that leave one, two or three rows in the last group, against numpy.
 
 Tolerance: a sum of n products in any order is within n u sum |m x| of the exact
@@ -15,9 +15,9 @@ pytestmark = pytest.mark.gpu
 U = 2.0 ** -53
 
 
-@pytest.mark.parametrize("sizes,vec", [([130] * 80, 1), ([130] * 83, 1), ([129] * 84, 0), ([131, 1, 2, 3] * 30, 0),
-                                       ([306] * 36, 1), ([306, 2, 64] * 13, 1), ([1206] * 9, 1), ([1205] * 9, 0),
-                                       ([5] * 2200, 0), ([2] * 6000, 1)])
+@pytest.mark.parametrize("sizes,vec", [([130] * 57, 1), ([130] * 58, 1), ([129] * 58, 0), ([131, 1, 2, 3] * 30, 0),
+                                       ([306] * 24, 1), ([306, 2, 64] * 13, 1), ([1206] * 7, 1), ([1205] * 7, 0),
+                                       ([5] * 1700, 0), ([2] * 6000, 1)])
 def test_products_match_numpy(sizes, vec):
     from fiber3d_b200 import _lib
     rng = np.random.default_rng(len(sizes))
